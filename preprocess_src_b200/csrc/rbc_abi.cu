@@ -386,13 +386,15 @@ void initial_volume(const rbc_handle *h, const CellGroup &g, const int *tri, con
     }
 }
 
-// Surface patches for the spread kernel: recursive coordinate bisection of the
-// first cell's initial vertex positions (split along the widest axis at the
-// median until a patch has at most 512 vertices).  The same vertex sets serve
-// every cell, since all cells share the mesh and a compact patch of the surface
-// stays compact as the membrane moves.  Also a lane stride per patch, near
-// 0.618 of its size and coprime with it, that scatters neighbours across lanes.
-void surface_patches(int V, const double *xr, std::vector<int> &off, std::vector<int> &vtx, std::vector<int> &stride)
+// Surface patches for the spread and advection kernels: recursive coordinate
+// bisection of the first cell's initial vertex positions (split along the
+// widest axis at the median until a patch has at most `most` vertices).  The
+// same vertex sets serve every cell, since all cells share the mesh and a
+// compact patch of the surface stays compact as the membrane moves.  Also a
+// lane stride per patch, near 0.618 of its size and coprime with it, that
+// scatters neighbours across lanes.
+void surface_patches(int V, int most, const double *xr, std::vector<int> &off, std::vector<int> &vtx,
+                     std::vector<int> &stride)
 {
     vtx.resize(V);
     for (int i = 0; i < V; i++) vtx[i] = i;
@@ -402,7 +404,7 @@ void surface_patches(int V, const double *xr, std::vector<int> &off, std::vector
     while (!stack.empty()) {
         auto [b, e] = stack.back();
         stack.pop_back();
-        if (e - b <= MAX_PATCH_VERTICES) { leaves.push_back({b, e}); continue; }
+        if (e - b <= most) { leaves.push_back({b, e}); continue; }
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
         for (int k = b; k < e; k++)
             for (int d = 0; d < 3; d++) { lo[d] = std::min(lo[d], xr[3 * vtx[k] + d]); hi[d] = std::max(hi[d], xr[3 * vtx[k] + d]); }
@@ -423,6 +425,28 @@ void surface_patches(int V, const double *xr, std::vector<int> &off, std::vector
         while (std::gcd(s, n) != 1) s += 2;
         stride.push_back(s);
     }
+}
+
+// Most vertices of a patch for a population of ncell cells of V vertices.  A
+// block of either kernel takes about 75 ns per vertex of its patch however few
+// blocks run (latency: a few warps per multiprocessor), so a population with
+// few cells is cut into more patches, down to 64 vertices (one pass of the
+// advection's 64 vertices per block), until there are two blocks per
+// multiprocessor.  One cell of 642 vertices in 2, 8, 16 and 32 patches: spread
+// 25, 15.1, 13.1 and 12.9 us, advection 27, 12.9, 11.0 and 10.8 us (events,
+// about 3 us of launch in each), step 71, 46.6, 42.3 and 43.3 us; 9 such cells
+// 74, 52.0, 49.3 and 51.6 us a step; six cells across a periodic x 146, 99, 95
+// and 96 us.  200 cells of 2562 vertices keep 8 patches each.
+int patch_vertices(int ncell, int V, int sms)
+{
+    auto patches = [&](int most) {
+        long long n = 1;
+        for (int v = V; v > most; v = (v + 1) / 2) n *= 2;
+        return n;
+    };
+    int most = MAX_PATCH_VERTICES;
+    while (most > MIN_PATCH_VERTICES && ncell * patches(most) < 2LL * sms) most /= 2;
+    return most;
 }
 
 // Edge-neighbour visits of fourpoint_bend (stress.cu:448-578, cel->ec from
@@ -1307,9 +1331,9 @@ int batch_build(rbc_batch *b)
 
 // Host-side setup of one cell population from its mesh (init2.cu:258-400,
 // volume_correction.cu:427-450): link tables, reference metric, V0 and
-// centroids, surface patches, bending visits.
+// centroids, bending visits.
 struct GroupPrep {
-    std::vector<int> off, packed, poff, pvtx, pstride;
+    std::vector<int> off, packed;
     std::vector<int16_t> nbr6, nbrp6;
     std::vector<int> vord;
     std::vector<double> vol0, gx, xs;
@@ -1324,8 +1348,6 @@ int prepare_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, GroupPrep &
     c.nv = (long long)c.ncell * c.V; c.ne = (long long)c.ncell * c.E;
     int rc = build_topology(h, c, mesh->tri, pp.off, pp.packed, pp.nbr6, pp.nbrp6, pp.vord);
     if (rc) return rc;
-    surface_patches(c.V, mesh->xr, pp.poff, pp.pvtx, pp.pstride);
-    c.npatch = (int)pp.poff.size() - 1;
     reference_metric(c, mesh->tri, mesh->xr, pp.gref);
     initial_volume(h, c, mesh->tri, mesh->xr, pp.vol0, pp.gx);
     pp.xs.resize(3 * c.nv);
@@ -1336,10 +1358,13 @@ int prepare_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, GroupPrep &
     return RBC_OK;
 }
 
-// device arrays of one cell population
+// device arrays of one cell population, and its surface patches
 int upload_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, const GroupPrep &pp)
 {
     int rc;
+    std::vector<int> poff, pvtx, pstride;
+    surface_patches(c.V, patch_vertices(c.ncell, c.V, h->sms), mesh->xr, poff, pvtx, pstride);
+    c.npatch = (int)poff.size() - 1;
 #define TRYG(x) do { if ((rc = (x))) return rc; } while (0)
     TRYG(dalloc(h, &c.X, 3 * c.nv)); TRYG(dalloc(h, &c.Xd, 3 * c.nv)); TRYG(dalloc(h, &c.gref, c.ne));
     CK(cudaMalloc(&c.erec, (size_t)c.ne * 12 * (h->p.membrane_fp64 ? sizeof(double) : sizeof(float))));
@@ -1355,8 +1380,8 @@ int upload_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, const GroupP
         TRYG(dalloc(h, &c.cs0, pp.cs0.size()));
         CK(cudaMemcpy(c.cs0, pp.cs0.data(), sizeof(double2) * pp.cs0.size(), cudaMemcpyHostToDevice));
     }
-    TRYG(dalloc(h, &c.patch_off, pp.poff.size())); TRYG(dalloc(h, &c.patch_vtx, pp.pvtx.size()));
-    TRYG(dalloc(h, &c.patch_stride, pp.pstride.size()));
+    TRYG(dalloc(h, &c.patch_off, poff.size())); TRYG(dalloc(h, &c.patch_vtx, pvtx.size()));
+    TRYG(dalloc(h, &c.patch_stride, pstride.size()));
     TRYG(dalloc(h, &c.vol0, c.ncell)); TRYG(dalloc(h, &c.gx, 3 * c.ncell));
     TRYG(dalloc(h, &c.vol_out, c.ncell)); TRYG(dalloc(h, &c.area_out, c.ncell)); TRYG(dalloc(h, &c.cen_out, 3 * c.ncell));
 #undef TRYG
@@ -1371,9 +1396,9 @@ int upload_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, const GroupP
     CK(cudaMemcpy(c.nbr, pp.nbr6.data(), 2 * 6 * c.V, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.nbrp, pp.nbrp6.data(), 2 * 6 * c.V, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.vord, pp.vord.data(), 4 * c.V, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c.patch_off, pp.poff.data(), 4 * pp.poff.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c.patch_vtx, pp.pvtx.data(), 4 * pp.pvtx.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c.patch_stride, pp.pstride.data(), 4 * pp.pstride.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(c.patch_off, poff.data(), 4 * poff.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(c.patch_vtx, pvtx.data(), 4 * pvtx.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(c.patch_stride, pstride.data(), 4 * pstride.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.vol0, pp.vol0.data(), 8 * c.ncell, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.gx, pp.gx.data(), 8 * 3 * c.ncell, cudaMemcpyHostToDevice));
     return RBC_OK;

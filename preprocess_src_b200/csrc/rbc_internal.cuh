@@ -245,8 +245,10 @@ int vof_cg_blocks();
 
 
 
-// Surface patches (spread and advection work units) hold at most this many vertices.
+// Surface patches (spread and advection work units) hold at most this many vertices,
+// and a population with few cells is not cut into patches of fewer than about half MIN.
 constexpr int MAX_PATCH_VERTICES = 512;
+constexpr int MIN_PATCH_VERTICES = 64;
 
 struct SpreadArgs {
     const double *X; long long nv; int V, ncell;
