@@ -971,6 +971,7 @@ VolumeArgs volume_args(rbc_handle *h, CellGroup &g, int correct)
     a.V = g.V; a.E = g.E; a.ncell = g.ncell;
     a.flags = h->d_flags(); a.vc_max = h->d_vcmax(); a.vc_last = h->d_vclast();
     a.correct = correct;
+    a.cache_normals = volume_caches_normals(g.V);
     return a;
 }
 

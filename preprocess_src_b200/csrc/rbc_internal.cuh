@@ -360,7 +360,9 @@ struct VolumeArgs {
     int V, E, ncell;
     int *flags, *vc_max, *vc_last;
     int correct;              // 0: metrics only (volume, area, centroid), positions untouched
+    int cache_normals;        // the block's shared memory holds the cell's unit normals (volume_caches_normals)
 };
+bool volume_caches_normals(int V);
 int  volume_smem_bytes(int V);
 void launch_volume(const Geom &g, const VolumeArgs &a, cudaStream_t s);
 

@@ -16,12 +16,18 @@
 
 namespace rbc {
 
+// threads of a block: one vertex (two elements) each for cells of up to 1024
+// vertices, so small cells meet fewer warps at each barrier and reduction
 constexpr int VOL_THREADS = 1024;
+static int volume_threads(int V) { return V >= VOL_THREADS ? VOL_THREADS : (V + 31) / 32 * 32; }
 constexpr double COEFF_VOL_CHANGE = 0.1;   // volume_correction.cu:14
 constexpr double VC_EPS = 1.0e-3;          // volume_correction.cu:15, percent
 constexpr int VC_ITRMAX = 1000;            // volume_correction.cu:487
 
-int volume_smem_bytes(int V) { return 24 * V; }
+// positions [3][V], then (where the block's shared memory holds them) unit normals [3][E], E = 2 V - 4
+constexpr int VOL_SMEM_MAX = 224 * 1024;
+bool volume_caches_normals(int V) { return 24 * (3 * V - 4) <= VOL_SMEM_MAX; }
+int volume_smem_bytes(int V) { return volume_caches_normals(V) ? 24 * (3 * V - 4) : 24 * V; }
 
 // block sums of K values at once: per value a warp butterfly, then the warps' sums in warp order
 template <int K>
@@ -55,9 +61,10 @@ __device__ __forceinline__ void ele_measure(const double *__restrict__ p, int V,
     tri_measure(A, B, C, s18v, s2a);
 }
 
-// unit normal, area and volume contribution of local element e (CalcEleNormal_GPU)
+// unit normal of local element e (CalcEleNormal_GPU), and its tri_measure when it is asked for
+template <bool MEASURE>
 __device__ __forceinline__ void ele_normal(const double *__restrict__ p, int V, const int *__restrict__ tri, int e,
-                                           double n[3], double &dS, double &vt)
+                                           double n[3], double &s18v, double &s2a)
 {
     const int na = __ldg(&tri[3 * e]), nb = __ldg(&tri[3 * e + 1]), nc = __ldg(&tri[3 * e + 2]);
     const double ax = p[na], ay = p[V + na], az = p[2 * V + na];
@@ -67,10 +74,12 @@ __device__ __forceinline__ void ele_normal(const double *__restrict__ p, int V, 
     const double v2x = cx - ax, v2y = cy - ay, v2z = cz - az;
     const double c0 = v1y * v2z - v1z * v2y, c1 = v1z * v2x - v1x * v2z, c2 = v1x * v2y - v1y * v2x;
     const double nc_ = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
-    n[0] = c0 / nc_; n[1] = c1 / nc_; n[2] = c2 / nc_;
-    dS = nc_ / 2.0;
-    const double rx = (ax + bx + cx) / 3.0, ry = (ay + by + cy) / 3.0, rz = (az + bz + cz) / 3.0;
-    vt = 1.0 / 3.0 * (rx * n[0] + ry * n[1] + rz * n[2]) * dS;
+    const double inv = 1.0 / nc_;
+    n[0] = c0 * inv; n[1] = c1 * inv; n[2] = c2 * inv;
+    if (MEASURE) {
+        s2a += nc_;
+        s18v += (ax + bx + cx) * c0 + (ay + by + cy) * c1 + (az + bz + cz) * c2;
+    }
 }
 
 // cell: the block's cell, blockIdx.x of a one-population launch
@@ -106,13 +115,30 @@ __device__ __forceinline__ void volume_body(const Geom &g, const VolumeArgs &a, 
     }
     __syncthreads();
 
+    // The move of a vertex needs the unit normals of its six elements.  They are
+    // formed once per element, in the measuring pass of the positions they belong to
+    // (from the second pass on: most calls move nothing and need none), and kept in
+    // shared memory: the FP64 square roots and divisions per move fall from 3 E to E,
+    // and since a move then reads only normals it updates the positions in place.
+    // Calls with one to ten moves, before and after (events): six cells of 642 vertices 81
+    // -> 47 us, 20 of 2562 and 4 of 162 55.5 -> 39, 200 of 2562 86 -> 68, one of 642 24 -> 19.6.
     const double V0 = a.correct ? a.vol0[cell] : 0.0;
+    double *nrm = p + 3 * (size_t)V;   // [3][E] where cached
+    const bool cached = a.cache_normals != 0;
     double vol = 0.0, area = 0.0;
     int it = 0;
     for (;;) {
         double s[2] = {0.0, 0.0};
+        if (cached && it > 0) {
+            for (int e = tid; e < E; e += T) {
+                double n[3];
+                ele_normal<true>(p, V, a.tri, e, n, s[0], s[1]);
+                nrm[e] = n[0]; nrm[E + e] = n[1]; nrm[2 * E + e] = n[2];
+            }
+        } else {
 #pragma unroll 2
-        for (int e = tid; e < E; e += T) ele_measure(p, V, a.tri, e, s[0], s[1]);
+            for (int e = tid; e < E; e += T) ele_measure(p, V, a.tri, e, s[0], s[1]);
+        }
         block_sum_k<2>(s, red);
         vol = s[0] / 18.0;
         area = s[1] / 2.0;
@@ -120,30 +146,50 @@ __device__ __forceinline__ void volume_body(const Geom &g, const VolumeArgs &a, 
         it++;
         if (fabs(vol - V0) / V0 * 100.0 < VC_EPS) break;
         const double lambda = 18.0 * (vol - V0) / area;
-        double disp[4][3];
-        for (int m = 0; m < 4; m++) {
-            const int v = tid + m * T;
-            disp[m][0] = disp[m][1] = disp[m][2] = 0.0;
-            if (v >= V) continue;
-            const int k0 = __ldg(&a.v2e_off[v]), k1 = __ldg(&a.v2e_off[v + 1]);
-            const int nne = k1 - k0;
-            double nn0 = 0.0, nn1 = 0.0, nn2 = 0.0;
-            for (int k = k0; k < k1; k++) {
-                double n[3], dS, vt;
-                ele_normal(p, V, a.tri, v2e_elem(__ldg(&a.v2e[k])), n, dS, vt);
-                nn0 += n[0] / nne; nn1 += n[1] / nne; nn2 += n[2] / nne;
+        const double move = -lambda / 6.0 * COEFF_VOL_CHANGE;
+        if (cached) {
+            if (it == 1) {
+                for (int e = tid; e < E; e += T) {
+                    double n[3], u0, u1;
+                    ele_normal<false>(p, V, a.tri, e, n, u0, u1);
+                    nrm[e] = n[0]; nrm[E + e] = n[1]; nrm[2 * E + e] = n[2];
+                }
+                __syncthreads();
             }
-            disp[m][0] = -lambda / 6.0 * nn0 * COEFF_VOL_CHANGE;
-            disp[m][1] = -lambda / 6.0 * nn1 * COEFF_VOL_CHANGE;
-            disp[m][2] = -lambda / 6.0 * nn2 * COEFF_VOL_CHANGE;
+            for (int v = tid; v < V; v += T) {
+                const int k0 = __ldg(&a.v2e_off[v]), k1 = __ldg(&a.v2e_off[v + 1]);
+                double n0 = 0.0, n1 = 0.0, n2 = 0.0;
+                for (int k = k0; k < k1; k++) {
+                    const int e = v2e_elem(__ldg(&a.v2e[k]));
+                    n0 += nrm[e]; n1 += nrm[E + e]; n2 += nrm[2 * E + e];
+                }
+                const double m = move / (double)(k1 - k0);
+                p[v] += m * n0; p[V + v] += m * n1; p[2 * V + v] += m * n2;
+            }
+            __syncthreads();
+        } else {   // a cell too large for the normals: each vertex forms those of its elements
+            double disp[4][3];
+            for (int m = 0; m < 4; m++) {
+                const int v = tid + m * T;
+                disp[m][0] = disp[m][1] = disp[m][2] = 0.0;
+                if (v >= V) continue;
+                const int k0 = __ldg(&a.v2e_off[v]), k1 = __ldg(&a.v2e_off[v + 1]);
+                for (int k = k0; k < k1; k++) {
+                    double n[3], u0, u1;
+                    ele_normal<false>(p, V, a.tri, v2e_elem(__ldg(&a.v2e[k])), n, u0, u1);
+                    disp[m][0] += n[0]; disp[m][1] += n[1]; disp[m][2] += n[2];
+                }
+                const double w = move / (double)(k1 - k0);
+                for (int c = 0; c < 3; c++) disp[m][c] *= w;
+            }
+            __syncthreads();
+            for (int m = 0; m < 4; m++) {
+                const int v = tid + m * T;
+                if (v >= V) continue;
+                p[v] += disp[m][0]; p[V + v] += disp[m][1]; p[2 * V + v] += disp[m][2];
+            }
+            __syncthreads();
         }
-        __syncthreads();
-        for (int m = 0; m < 4; m++) {
-            const int v = tid + m * T;
-            if (v >= V) continue;
-            p[v] += disp[m][0]; p[V + v] += disp[m][1]; p[2 * V + v] += disp[m][2];
-        }
-        __syncthreads();
         if (it >= VC_ITRMAX) { if (tid == 0) atomicOr(a.flags, RBC_FLAG_VC_NOT_CONVERGED); break; }
     }
     // CalcCenter: vertex mean, wrapped into [zmin, zmax]; with a correction, the same pass
@@ -183,8 +229,7 @@ volume_kernel(const Geom g, const VolumeArgs a)
 void launch_volume(const Geom &g, const VolumeArgs &a, cudaStream_t s)
 {
     if (a.ncell <= 0) return;
-    const int smem = volume_smem_bytes(a.V);
-    launch_pdl(volume_kernel, dim3(a.ncell), dim3(VOL_THREADS), smem, s, g, a);
+    launch_pdl(volume_kernel, dim3(a.ncell), dim3(volume_threads(a.V)), volume_smem_bytes(a.V), s, g, a);
 }
 
 cudaError_t membrane_setup(int optin, int *max_bytes);
@@ -299,7 +344,7 @@ cudaError_t volume_fused_setup(int optin)
 void launch_volume_fused(const FusedLaunch &f, int V, cudaStream_t s)
 {
     if (f.nblocks > 0)
-        volume_fused_kernel<<<f.nblocks, VOL_THREADS, volume_smem_bytes(V), s>>>(f.dom, f.boff, f.ndom);
+        volume_fused_kernel<<<f.nblocks, volume_threads(V), volume_smem_bytes(V), s>>>(f.dom, f.boff, f.ndom);
 }
 
 }  // namespace rbc
