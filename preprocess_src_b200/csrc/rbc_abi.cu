@@ -123,6 +123,7 @@ struct rbc_handle {
     cudaEvent_t wave_done = nullptr, spread_done = nullptr;
     // the force reset beside the advection (capture only; on side2, idle by then)
     cudaEvent_t lbm_done = nullptr, reset_done = nullptr;
+    cudaEvent_t thinc_done = nullptr;   // the volume fraction's sweeps beside the advection (capture only; on side)
     int sms = 0;                                      // multiprocessors of the device
     int prio_high = 0;                                // greatest stream priority of the device
     long long launches = 0;
@@ -682,6 +683,7 @@ void free_all(rbc_handle *h)
     if (h->spread_done) cudaEventDestroy(h->spread_done);
     if (h->lbm_done) cudaEventDestroy(h->lbm_done);
     if (h->reset_done) cudaEventDestroy(h->reset_done);
+    if (h->thinc_done) cudaEventDestroy(h->thinc_done);
     if (h->side2) cudaStreamDestroy(h->side2);
     for (int k = 0; k < 4; k++) {
         if (h->imp_copied[k]) cudaEventDestroy(h->imp_copied[k]);
@@ -901,13 +903,13 @@ int launch_advect_stage(rbc_handle *h)
     return RBC_OK;
 }
 
-// thinc_wlic (thincwlic.cu:316-420) of every population's volume fraction
-int launch_thinc_stage(rbc_handle *h)
+// thinc_wlic (thincwlic.cu:316-420) of every population's volume fraction, on stream st
+int launch_thinc_stage(rbc_handle *h, cudaStream_t st)
 {
     for (int k = 0; k < h->ngroups; k++) {
         CellGroup &g = h->cg[k];
         if (!g.vf || g.ncell == 0) continue;
-        launch_thinc_wlic(h->geo, g.vf, h->vof_s1, h->vof_s2, h->uvr, h->mask2d, h->p.dt * h->p.M, h->stream);
+        launch_thinc_wlic(h->geo, g.vf, h->vof_s1, h->vof_s2, h->uvr, h->mask2d, h->p.dt * h->p.M, st);
         h->launches += 3;
         CK_LAUNCH();
     }
@@ -1065,10 +1067,17 @@ int enqueue_step(rbc_handle *h, StepForm form = STEP_WHOLE)
     CK(cudaStreamWaitEvent(h->side2, h->lbm_done, 0));
     if ((rc = launch_force_reset_stage(h, h->side2))) return rc;
     CK(cudaEventRecord(h->reset_done, h->side2));
+    // the volume fraction's sweeps (main.cu:94-95) read the same velocity as the
+    // advection and neither touches the other's data: on a branch of their own
+    if (h->vof()) {
+        CK(cudaStreamWaitEvent(h->side, h->lbm_done, 0));
+        if ((rc = launch_thinc_stage(h, h->side))) return rc;
+        CK(cudaEventRecord(h->thinc_done, h->side));
+    }
     if ((rc = launch_advect_stage(h))) return rc;
-    if ((rc = launch_thinc_stage(h))) return rc;   // main.cu:94-95
     if ((form == STEP_WHOLE || form == STEP_SUB_LAST) && (rc = launch_volume_stage(h, h->stream))) return rc;
     CK(cudaStreamWaitEvent(h->stream, h->reset_done, 0));
+    if (h->vof()) CK(cudaStreamWaitEvent(h->stream, h->thinc_done, 0));
     return RBC_OK;
 }
 
@@ -1563,6 +1572,7 @@ int rbc_create(const rbc_params *p, const rbc_mesh *mesh, const int *bc, rbc_han
             cudaEventCreateWithFlags(&h->spread_done, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&h->lbm_done, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&h->reset_done, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&h->thinc_done, cudaEventDisableTiming) != cudaSuccess ||
             cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) {
             h->err = "stream creation failed";
             return bail(RBC_ERR_CUDA);
@@ -2001,7 +2011,7 @@ int rbc_thinc_wlic(rbc_handle *h)
 {
     if (!h) return RBC_ERR_ARG;
     RBC_DEVICE_GUARD(h);
-    return launch_thinc_stage(h);
+    return launch_thinc_stage(h, h->stream);
 }
 
 int rbc_front_tracking(rbc_handle *h, int *iters)
@@ -2174,7 +2184,7 @@ int rbc_profile_steps(rbc_handle *h, int nsteps, double *kernel_ms)
         cudaEventRecord(ev[5], h->stream);
         if (!rc && last) rc = launch_advect_stage(h);
         cudaEventRecord(ev[6], h->stream);
-        if (!rc && last) rc = launch_thinc_stage(h);
+        if (!rc && last) rc = launch_thinc_stage(h, h->stream);
         if (!rc && h->vof() && (h->iter + s + 1) % h->p.vof_k == 0) rc = launch_front_tracking_stage(h);
         cudaEventRecord(ev[7], h->stream);
         if (!rc && last) rc = launch_volume_stage(h, h->stream);

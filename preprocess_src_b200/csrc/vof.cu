@@ -231,12 +231,15 @@ thinc_sweep_kernel(const Geom g, const double *__restrict__ vin, double *__restr
 
 // ---- front tracking -------------------------------------------------------
 
-// front_tracking_source2 (fronttrack.cu:351-455) for one triangle per thread
+// front_tracking_source2 (fronttrack.cu:351-455), four threads per triangle, one
+// z plane of its stencil each: a thread's 16 nodes of three FP64 atomics are a
+// serial chain, and a few cells' triangles alone do not fill the GPU (8 cells of
+// 1280 triangles took 52 us with one thread per triangle)
 __global__ void __launch_bounds__(VOF_THREADS)
 indicator_gradient_kernel(const Geom g, const double *__restrict__ X, long long nv, const int *__restrict__ tri,
                           int V, int E, int ncell, const uint32_t *__restrict__ mask2d, double *__restrict__ G)
 {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, e = t >> 2;
     if (e >= (long long)ncell * E) return;
     const int c = (int)(e / E), k = (int)(e - (long long)c * E);
     const long long base = (long long)c * V;
@@ -265,7 +268,7 @@ indicator_gradient_kernel(const Geom g, const double *__restrict__ X, long long 
     const int z1 = (int)floor(ztr / dx) - 1, z2 = (int)ceil(ztr / dx) + 1;
     const double inv64 = 1.0 / (64.0 * dx * dx * dx);
     double *Gx = G, *Gy = G + g.nint, *Gz = G + 2 * g.nint;
-    for (int iz = z1; iz <= z2; iz++) {
+    for (int iz = z1 + (int)(t & 3); iz <= z2; iz += 4) {
         if (iz < 0 || iz >= g.nzr) continue;
         const double zcos = 1.0 + cospi(((double)iz * dx - ztr) / (2.0 * dx));
         for (int iy = y1; iy <= y2; iy++) {
@@ -508,6 +511,81 @@ struct PcgArgs {
 
 constexpr double MG_OMEGA = 0.8;   // damped-Jacobi smoothing weight
 constexpr int MG_COARSE_SWEEPS = 40;
+constexpr int MG_COARSE_SMEM = 512;   // nodes of a coarsest level swept in shared memory (the coarsening's target)
+
+// The coarsest level: Jacobi sweeps from 0 in block 0.  Each sweep is a short
+// dependent step (seven loads, one barrier), so it runs from shared memory with
+// each thread's rows in registers.
+__device__ void coarse_sweeps(const MgLevel &C)
+{
+    __shared__ double sx[2][MG_COARSE_SMEM];
+    constexpr int PER = MG_COARSE_SMEM / CG_THREADS;
+    const unsigned nc = (unsigned)C.n, ncc = (unsigned)(C.nx * C.ny);
+    if (nc <= MG_COARSE_SMEM) {
+        double bb[PER], id[PER], cf[PER][6];
+        int nb[PER][6];
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            const unsigned i = threadIdx.x + k * CG_THREADS;
+            bb[k] = id[k] = 0.0;
+#pragma unroll
+            for (int m = 0; m < 6; m++) { cf[k][m] = 0.0; nb[k][m] = 0; }
+            if (i >= nc) continue;
+            const unsigned Z = i / ncc, rc = i - Z * ncc;
+            const int Y = (int)(rc / (unsigned)C.nx), X = (int)(rc - Y * (unsigned)C.nx);
+            sx[0][i] = 0.0;
+            const double inv = C.coef[6 * ncc + rc];
+            if (inv == 0.0) continue;
+            bb[k] = C.b[i]; id[k] = MG_OMEGA * inv;
+            const int xl = X > 0 ? X - 1 : C.nx - 1, xr = X < C.nx - 1 ? X + 1 : 0;
+            const int zm = Z == 0 ? C.nz - 1 : (int)Z - 1, zp = (int)Z == C.nz - 1 ? 0 : (int)Z + 1;
+            const int zo = (int)(Z * ncc);
+            cf[k][0] = C.coef[ncc + rc];     nb[k][0] = zo + Y * C.nx + xl;
+            cf[k][1] = C.coef[2 * ncc + rc]; nb[k][1] = zo + Y * C.nx + xr;
+            cf[k][2] = C.coef[3 * ncc + rc]; nb[k][2] = cf[k][2] != 0.0 ? zo + (Y - 1) * C.nx + X : 0;
+            cf[k][3] = C.coef[4 * ncc + rc]; nb[k][3] = cf[k][3] != 0.0 ? zo + (Y + 1) * C.nx + X : 0;
+            cf[k][4] = cf[k][5] = C.coef[5 * ncc + rc];
+            nb[k][4] = zm * (int)ncc + (int)rc; nb[k][5] = zp * (int)ncc + (int)rc;
+            // D^-1 D x = x: the sweep x + w D^-1 (b - A x) is (1 - w) x + w D^-1 (b - off x)
+        }
+        __syncthreads();
+        for (int sw = 0; sw < MG_COARSE_SWEEPS; sw++) {
+            const double *src = sx[sw & 1];
+            double *dst = sx[(sw + 1) & 1];
+#pragma unroll
+            for (int k = 0; k < PER; k++) {
+                const unsigned i = threadIdx.x + k * CG_THREADS;
+                if (i >= nc) continue;
+                double t = bb[k];
+#pragma unroll
+                for (int m = 0; m < 6; m++) t -= cf[k][m] * src[nb[k][m]];
+                dst[i] = id[k] != 0.0 ? (1.0 - MG_OMEGA) * src[i] + id[k] * t : 0.0;
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            const unsigned i = threadIdx.x + k * CG_THREADS;
+            if (i < nc) C.y[i] = sx[MG_COARSE_SWEEPS & 1][i];
+        }
+        return;
+    }
+    // a lattice whose extents do not coarsen that far: from global memory (x and y alternate)
+    for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) C.y[i] = 0.0;
+    __syncthreads();
+    double *src = C.y, *dst = C.x;
+    for (int sw = 0; sw < MG_COARSE_SWEEPS; sw++) {
+        for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) {
+            const unsigned Z = i / ncc, rc = i - Z * ncc, Y = rc / (unsigned)C.nx, X = rc - Y * (unsigned)C.nx;
+            const double id = C.coef[6 * ncc + rc];
+            dst[i] = id != 0.0 ? src[i] + MG_OMEGA * (C.b[i] - apply_level(C, src, i, (int)X, (int)Y, (int)Z)) * id : 0.0;
+        }
+        __syncthreads();
+        double *t = src; src = dst; dst = t;
+    }
+    if (src != C.y)
+        for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) C.y[i] = src[i];
+}
 
 // z = M r: one symmetric V-cycle (one damped-Jacobi sweep from 0 before and
 // one after the coarse correction, the coarsest level by Jacobi sweeps in
@@ -515,8 +593,14 @@ constexpr int MG_COARSE_SWEEPS = 40;
 // pre-smoothed iterate x = w D^-1 b is never stored: the restriction of its
 // residual and the post-smoothing (with x = w D^-1 b + P y_coarse) evaluate
 // it at the stencil's nodes, so each level costs one pass and one barrier on
-// the way down and one on the way up.
-__device__ void vcycle(cg::grid_group &grid, const PcgArgs &a, unsigned first, unsigned stride)
+// the way down and one on the way up.  Short passes, the barriers and the coarsest
+// level's serial sweeps bound it: 96 x 48 x 48 nodes 170 -> 56 us per CG iteration,
+// 33 x 24 x 20 150 -> 47, 256 x 128 x 128 410 -> 320 (with the coarsest level swept
+// from global memory, the restriction at one thread per coarse node and two more
+// grid barriers -> as here; 1, 2 and 3 blocks per multiprocessor: 66, 57 and 56 us on
+// the first, 690, 402 and 320 on the last).  Returns the thread's share of r . z; the
+// caller's grid sum is the barrier after the last pass.
+__device__ double vcycle(cg::grid_group &grid, const PcgArgs &a, unsigned first, unsigned stride)
 {
     const int L = a.mg.nlev;
     for (int l = 0; l < L - 1; l++) {
@@ -525,43 +609,30 @@ __device__ void vcycle(cg::grid_group &grid, const PcgArgs &a, unsigned first, u
         const double *fb = F.b, *fc = F.coef;
         auto xpre = [fb, fc, ncf](unsigned j, unsigned c, int, int, int) { return MG_OMEGA * fb[j] * fc[6 * ncf + c]; };
         const unsigned nc = (unsigned)C.n, ncc = (unsigned)(C.nx * C.ny);
-        for (unsigned I = first; I < nc; I += stride) {
-            const unsigned Z = I / ncc, rc = I - Z * ncc, Y = rc / (unsigned)C.nx, X = rc - Y * (unsigned)C.nx;
+        // eight lanes per coarse node, one fine node of its block each (bit 0, 1, 2 of the lane:
+        // x, y, z), then a sum over the lanes: the fine level's parallelism instead of the coarse one's
+        const unsigned sub = first & 7u;
+        const int dx = (int)(sub & 1u), dy = (int)((sub >> 1) & 1u), dz = (int)(sub >> 2);
+        for (unsigned I0 = (first & ~31u) >> 3; I0 < nc; I0 += stride >> 3) {   // uniform over the warp
+            const unsigned I = I0 + ((first & 31u) >> 3);
             double s = 0.0;
-            for (int dz = 0; dz < F.bz; dz++)
-                for (int dy = 0; dy < F.by; dy++)
-                    for (int dx = 0; dx < F.bx; dx++) {
-                        const int x = (int)X * F.bx + dx, y = (int)Y * F.by + dy, z = (int)Z * F.bz + dz;
-                        if (x >= F.nx || y >= F.ny) continue;
-                        const unsigned col = (unsigned)(y * F.nx + x), i = (unsigned)z * ncf + col;
-                        if (fc[col] == 0.0) continue;
-                        s += fb[i] - apply_level_fn(F, x, y, z, xpre);
-                    }
-            C.b[I] = s;
-        }
-        grid.sync();
-    }
-    {   // coarsest level: Jacobi sweeps from 0 in block 0 (x and y alternate)
-        const MgLevel &C = a.mg.lev[L - 1];
-        if (blockIdx.x == 0) {
-            const unsigned nc = (unsigned)C.n, ncc = (unsigned)(C.nx * C.ny);
-            for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) C.y[i] = 0.0;
-            __syncthreads();
-            double *src = C.y, *dst = C.x;
-            for (int sw = 0; sw < MG_COARSE_SWEEPS; sw++) {
-                for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) {
-                    const unsigned Z = i / ncc, rc = i - Z * ncc, Y = rc / (unsigned)C.nx, X = rc - Y * (unsigned)C.nx;
-                    const double id = C.coef[6 * ncc + rc];
-                    dst[i] = id != 0.0 ? src[i] + MG_OMEGA * (C.b[i] - apply_level(C, src, i, (int)X, (int)Y, (int)Z)) * id : 0.0;
+            if (I < nc && dx < F.bx && dy < F.by && dz < F.bz) {
+                const unsigned Z = I / ncc, rc = I - Z * ncc, Y = rc / (unsigned)C.nx, X = rc - Y * (unsigned)C.nx;
+                const int x = (int)X * F.bx + dx, y = (int)Y * F.by + dy, z = (int)Z * F.bz + dz;
+                if (x < F.nx && y < F.ny) {
+                    const unsigned col = (unsigned)(y * F.nx + x);
+                    if (fc[col] != 0.0) s = fb[(unsigned)z * ncf + col] - apply_level_fn(F, x, y, z, xpre);
                 }
-                __syncthreads();
-                double *t = src; src = dst; dst = t;
             }
-            if (src != C.y)
-                for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) C.y[i] = src[i];
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (I < nc && sub == 0u) C.b[I] = s;
         }
         grid.sync();
     }
+    if (blockIdx.x == 0) coarse_sweeps(a.mg.lev[L - 1]);
+    grid.sync();
+    double lrz = 0.0;
     for (int l = L - 2; l >= 0; l--) {
         const MgLevel &F = a.mg.lev[l], &C = a.mg.lev[l + 1];
         const unsigned nf = (unsigned)F.n, ncf = (unsigned)(F.nx * F.ny), ncc = (unsigned)(C.nx * C.ny);
@@ -576,16 +647,23 @@ __device__ void vcycle(cg::grid_group &grid, const PcgArgs &a, unsigned first, u
         for (unsigned i = first; i < nf; i += stride) {
             const unsigned z = i / ncf, rc = i - z * ncf, y = rc / (unsigned)F.nx, x = rc - y * (unsigned)F.nx;
             const double id = fc[6 * ncf + rc];
-            F.y[i] = id != 0.0 ? xcor(i, rc, (int)x, (int)y, (int)z)
-                                     + MG_OMEGA * (fb[i] - apply_level_fn(F, (int)x, (int)y, (int)z, xcor)) * id
-                               : 0.0;
+            const double bi = fb[i];
+            const double yi = id != 0.0 ? xcor(i, rc, (int)x, (int)y, (int)z)
+                                              + MG_OMEGA * (bi - apply_level_fn(F, (int)x, (int)y, (int)z, xcor)) * id
+                                        : 0.0;
+            F.y[i] = yi;
+            if (l == 0) lrz += bi * yi;
         }
-        grid.sync();
+        if (l > 0) grid.sync();
     }
+    return lrz;
 }
 
 constexpr int PCG_BLOCKS_PER_SM = 3;
 
+// Preconditioned CG with r . z summed in the V-cycle's last pass, and A p by the
+// recurrence q = A z + beta q in the pass that updates p: three grid sums (each
+// a grid barrier) per iteration beside the V-cycle's own barriers, none for p.
 __global__ void __launch_bounds__(CG_THREADS, PCG_BLOCKS_PER_SM)
 indicator_pcg_kernel(const PcgArgs a)
 {
@@ -596,7 +674,9 @@ indicator_pcg_kernel(const PcgArgs a)
     double lr = 0.0, lb = 0.0;
     for (unsigned i = first; i < n; i += stride) {
         const unsigned z = i / ncol, rc = i - z * ncol, y = rc / (unsigned)L0.nx, x = rc - y * (unsigned)L0.nx;
-        if (L0.coef[rc] == 0.0) { a.x[i] = 0.0; a.r[i] = 0.0; a.p[i] = 0.0; continue; }
+        a.p[i] = 0.0;
+        a.q[i] = 0.0;
+        if (L0.coef[rc] == 0.0) { a.x[i] = 0.0; a.r[i] = 0.0; continue; }
         const double ri = a.b[i] - apply_level(L0, a.x, i, (int)x, (int)y, (int)z);
         a.r[i] = ri;
         lr += ri * ri;
@@ -607,20 +687,23 @@ indicator_pcg_kernel(const PcgArgs a)
     grid_sum2(grid, a.partial, bank, lr, lb, rr, bb);
     bank ^= 1;
     int it = 0;
-    if (bb > 0.0 && !(sqrt(rr / bb) < a.tol)) {
-        vcycle(grid, a, first, stride);   // z = M r (level 0's y)
-        double lrz = 0.0;
-        for (unsigned i = first; i < n; i += stride) { a.p[i] = L0.y[i]; lrz += a.r[i] * L0.y[i]; }
-        double rz, unused;
-        grid_sum2(grid, a.partial, bank, lrz, 0.0, rz, unused);
-        bank ^= 1;
-        while (it < a.itrmax) {
+    if (bb > 0.0) {
+        double rz = 0.0, unused;
+        while (it < a.itrmax && !(sqrt(rr / bb) < a.tol)) {
+            const double lrz = vcycle(grid, a, first, stride);   // z = M r (level 0's y)
+            double rz_new;
+            grid_sum2(grid, a.partial, bank, lrz, 0.0, rz_new, unused);
+            bank ^= 1;
+            const double beta = it > 0 ? rz_new / rz : 0.0;
+            rz = rz_new;
             double lpq = 0.0;
             for (unsigned i = first; i < n; i += stride) {
                 const unsigned z = i / ncol, rc = i - z * ncol, y = rc / (unsigned)L0.nx, x = rc - y * (unsigned)L0.nx;
-                const double qi = apply_level(L0, a.p, i, (int)x, (int)y, (int)z);
+                const double pi = L0.y[i] + beta * a.p[i];
+                const double qi = apply_level(L0, L0.y, i, (int)x, (int)y, (int)z) + beta * a.q[i];
+                a.p[i] = pi;
                 a.q[i] = qi;
-                lpq += a.p[i] * qi;
+                lpq += pi * qi;
             }
             double pq;
             grid_sum2(grid, a.partial, bank, lpq, 0.0, pq, unused);
@@ -636,17 +719,6 @@ indicator_pcg_kernel(const PcgArgs a)
             grid_sum2(grid, a.partial, bank, lrr, 0.0, rr, unused);
             bank ^= 1;
             it++;
-            if (sqrt(rr / bb) < a.tol) break;
-            vcycle(grid, a, first, stride);
-            double lrz2 = 0.0;
-            for (unsigned i = first; i < n; i += stride) lrz2 += a.r[i] * L0.y[i];
-            double rz_new;
-            grid_sum2(grid, a.partial, bank, lrz2, 0.0, rz_new, unused);
-            bank ^= 1;
-            const double beta = rz_new / rz;
-            rz = rz_new;
-            for (unsigned i = first; i < n; i += stride) a.p[i] = L0.y[i] + beta * a.p[i];
-            grid.sync();
         }
     }
     if (bb == 0.0)
@@ -786,7 +858,7 @@ cudaError_t launch_front_tracking(const Geom &g, const FrontArgs &a, cudaStream_
 {
     cudaError_t e = cudaMemsetAsync(a.G, 0, sizeof(double) * 3 * (size_t)g.nint, s);
     if (e != cudaSuccess) return e;
-    const long long ntri = (long long)a.ncell * a.E;
+    const long long ntri = 4LL * a.ncell * a.E;   // four threads each
     if (ntri > 0)
         indicator_gradient_kernel<<<(unsigned)((ntri + VOF_THREADS - 1) / VOF_THREADS), VOF_THREADS, 0, s>>>(
             g, a.X, a.nv, a.tri, a.V, a.E, a.ncell, a.mask2d, a.G);
