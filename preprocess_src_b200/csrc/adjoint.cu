@@ -12,10 +12,10 @@
 // its inputs.  The collision of one node is differentiated by hand in reverse
 // mode, and pull streaming with half-way bounce-back, which reads every fluid
 // slot exactly once, is reversed as a conflict-free push in the same kernel.
-// The Skalak loads of one element and the normal / area / volume of one
-// triangle are written once as templates on the scalar type; a forward-mode
-// dual number (value plus one derivative) seeded on one input at a time gives
-// one column of their Jacobian, which is contracted with the output adjoint.
+// The Skalak loads of one element are written once as a template on the scalar
+// type; a forward-mode dual number (value plus one derivative) seeded on one input
+// at a time gives one column of their Jacobian, which is contracted with the
+// output adjoint.  The normal, area and volume of a triangle are reversed by hand.
 // Spreading and interpolation are each other's transpose (plus the derivative
 // of the delta weights with respect to the vertex position); RK4 runs its
 // stages backwards; the mass-matrix solve M q = b (M symmetric) is reversed
@@ -257,41 +257,45 @@ __device__ __forceinline__ bool sane_pos(const Geom &g, double px, double py, do
 
 constexpr int VTX_ADJ_THREADS = 128;   // four vertices per CTA, one warp each
 
+// One RK stage's stencil with the velocity at the lane's two nodes, kept from the
+// replay of the stages for their reversal: the FP64 sines and cosines, the weights
+// and the loads are the cost of a stage, and each is needed twice (642 vertices:
+// 14.4 -> 12.3 us).
+struct StageStencil {
+    LaneStencil s;
+    float3 q[2];
+};
+
 // Velocity of the frozen field at p as the forward advection interpolates it
 // (every lane returns the same sum).
 __device__ __forceinline__ void warp_interp(const Geom &g, const float4 *__restrict__ uvr, const double p[3], int lane,
-                                            double u[3]) {
-    LaneStencil s;
-    lane_stencil(g, p[0], p[1], p[2], lane, s);
+                                            StageStencil &st, double u[3]) {
+    lane_stencil(g, p[0], p[1], p[2], lane, st.s);
     double u0 = 0.0, u1 = 0.0, u2 = 0.0;
 #pragma unroll
-    for (int h = 0; h < 2; h++)
-        if (s.n[h] >= 0) {
-            const float4 q = __ldg(&uvr[s.n[h]]);
-            u0 += s.w[h] * q.x; u1 += s.w[h] * q.y; u2 += s.w[h] * q.z;
-        }
+    for (int h = 0; h < 2; h++) {
+        const float4 q = st.s.n[h] >= 0 ? __ldg(&uvr[st.s.n[h]]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        st.q[h] = make_float3(q.x, q.y, q.z);
+        u0 += st.s.w[h] * q.x; u1 += st.s.w[h] * q.y; u2 += st.s.w[h] * q.z;
+    }
     u[0] = warp_sum(u0); u[1] = warp_sum(u1); u[2] = warp_sum(u2);
 }
 
-// Adjoint of one interpolation at p with output adjoint kb: adds w_n kb to
-// the velocity adjoint of each stencil node; returns in pb (every lane) the
+// Adjoint of one interpolation with output adjoint kb: adds w_n kb to the
+// velocity adjoint of each stencil node; returns in pb (every lane) the
 // position adjoint sum_n (d w_n / d p) (u_n . kb).
-__device__ __forceinline__ void warp_interp_adjoint(const Geom &g, const float4 *__restrict__ uvr,
-                                                    float *__restrict__ ubar, const double p[3], const double kb[3],
-                                                    int lane, double pb[3]) {
-    LaneStencil s;
-    lane_stencil(g, p[0], p[1], p[2], lane, s);
+__device__ __forceinline__ void warp_interp_adjoint(float *__restrict__ ubar, const StageStencil &st, const double kb[3],
+                                                    double pb[3]) {
     double b0 = 0.0, b1 = 0.0, b2 = 0.0;
 #pragma unroll
     for (int h = 0; h < 2; h++)
-        if (s.n[h] >= 0) {
-            const long long n = s.n[h];
-            const float4 q = __ldg(&uvr[n]);
-            atomicAdd(&ubar[4 * n + 0], (float)(s.w[h] * kb[0]));
-            atomicAdd(&ubar[4 * n + 1], (float)(s.w[h] * kb[1]));
-            atomicAdd(&ubar[4 * n + 2], (float)(s.w[h] * kb[2]));
-            const double uk = q.x * kb[0] + q.y * kb[1] + q.z * kb[2];
-            b0 += s.dw[h][0] * uk; b1 += s.dw[h][1] * uk; b2 += s.dw[h][2] * uk;
+        if (st.s.n[h] >= 0) {
+            const long long n = st.s.n[h];
+            atomicAdd(&ubar[4 * n + 0], (float)(st.s.w[h] * kb[0]));
+            atomicAdd(&ubar[4 * n + 1], (float)(st.s.w[h] * kb[1]));
+            atomicAdd(&ubar[4 * n + 2], (float)(st.s.w[h] * kb[2]));
+            const double uk = st.q[h].x * kb[0] + st.q[h].y * kb[1] + st.q[h].z * kb[2];
+            b0 += st.s.dw[h][0] * uk; b1 += st.s.dw[h][1] * uk; b2 += st.s.dw[h][2] * uk;
         }
     pb[0] = warp_sum(b0); pb[1] = warp_sum(b1); pb[2] = warp_sum(b2);
 }
@@ -307,20 +311,13 @@ advect_adjoint_kernel(const Geom g, const double *__restrict__ X, const float4 *
     const long long v = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (v >= nv) return;   // uniform over the warp
-    double p[4][3], k[3][3];
-    p[0][0] = X[v]; p[0][1] = X[nv + v]; p[0][2] = X[2 * nv + v];
-    if (!sane_pos(g, p[0][0], p[0][1], p[0][2])) {
+    const double p0[3] = {X[v], X[nv + v], X[2 * nv + v]};
+    if (!sane_pos(g, p0[0], p0[1], p0[2])) {
         if (lane == 0) {
             atomicOr(flags, RBC_FLAG_NONFINITE);
             X_bar[v] = X_bar[nv + v] = X_bar[2 * nv + v] = 0.0;
         }
         return;
-    }
-    const double hs[4] = {0.0, 0.5 * dtM, 0.5 * dtM, dtM};   // stage offsets (ibm.cu:474-498)
-    for (int s = 0; s < 3; s++) {
-        warp_interp(g, uvr, p[s], lane, k[s]);
-        // the forward adds the FP32 stage velocity to the FP64 position
-        for (int c = 0; c < 3; c++) p[s + 1][c] = p[0][c] + (double)(float)k[s][c] * hs[s + 1];
     }
     double xb[3], kb[4][3];
     for (int c = 0; c < 3; c++) {
@@ -328,15 +325,27 @@ advect_adjoint_kernel(const Geom g, const double *__restrict__ X, const float4 *
         xb[c] = a;   // Xa = X + dt (k1 + 2 k2 + 2 k3 + k4) / 6
         kb[0][c] = a * dtM / 6.0; kb[1][c] = a * dtM / 3.0; kb[2][c] = a * dtM / 3.0; kb[3][c] = a * dtM / 6.0;
     }
+    const double hs[4] = {0.0, 0.5 * dtM, 0.5 * dtM, dtM};   // stage offsets (ibm.cu:474-498)
+    StageStencil st[4];
+    double p[3] = {p0[0], p0[1], p0[2]};
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+        double k[3];
+        warp_interp(g, uvr, p, lane, st[s], k);
+        // the forward adds the FP32 stage velocity to the FP64 position
+        if (s < 3)
+            for (int c = 0; c < 3; c++) p[c] = p0[c] + (double)(float)k[c] * hs[s + 1];
+    }
+#pragma unroll
     for (int s = 3; s >= 0; s--) {
         double pb[3];
-        warp_interp_adjoint(g, uvr, ubar, p[s], kb[s], lane, pb);
+        warp_interp_adjoint(ubar, st[s], kb[s], pb);
         for (int c = 0; c < 3; c++) {
             xb[c] += pb[c];
             if (s > 0) kb[s - 1][c] += hs[s] * pb[c];   // p_s = X + h_s k_s-1
         }
     }
-    if (lane < 3) X_bar[(long long)lane * nv + v] = xb[lane];
+    if (lane < 3) X_bar[(long long)lane * nv + v] = lane == 0 ? xb[0] : lane == 1 ? xb[1] : xb[2];
 }
 
 // ---- spreading, reversed --------------------------------------------------
@@ -437,8 +446,6 @@ __device__ __forceinline__ void edges_of(const MembraneAdjArgs &a, long long vb,
     e2[0] = mimage_d(xs[ic] - xs[ia], a.LX); e2[1] = ys[ic] - ys[ia]; e2[2] = mimage_d(zs[ic] - zs[ia], a.LZ);
 }
 
-constexpr int MEM_ADJ_THREADS = 1024;
-
 // The forward solves M q = b per cell (b = element loads gathered per vertex,
 // M the P1 mass matrix) and sets Fv = -q ds (ds = one-ring area / 3).  Its
 // reverse, from Fv_bar: q_bar = -ds Fv_bar, ds_bar = -q . Fv_bar,
@@ -449,20 +456,20 @@ constexpr int MEM_ADJ_THREADS = 1024;
 // for the gather.
 
 // One CTA per cell: element areas (scratch[7 e]), rows of D^-1 M, q, ds_bar,
-// and lambda; writes lam, qv, dsb per vertex.
+// and lambda; writes lam, qv, dsb per vertex.  The solve runs as the forward's:
+// positions of the breadth-first order, rows and neighbours in registers, one
+// shared array per component.  One cell of 642 vertices: 27.9 -> 17.1 us against
+// neighbours, rows and four-float values read from shared memory every iteration.
 template <int VPT>
-__global__ void __launch_bounds__(MEM_ADJ_THREADS, 1)
+__global__ void __launch_bounds__(VPT >= 3 ? 896 : 1024, 1)
 membrane_adjoint_solve_kernel(const MembraneAdjArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int V = a.V, E = a.E, tid = threadIdx.x, T = blockDim.x;
-    float4 *dbuf = reinterpret_cast<float4 *>(smem);                    // [2][V]
-    float *coef = reinterpret_cast<float *>(smem + 32 * (size_t)V);     // [6][V]
-    int16_t *snbr = reinterpret_cast<int16_t *>(smem + 56 * (size_t)V); // [6][V]
+    float *dbuf = reinterpret_cast<float *>(smem);   // [2][3][V], by solve position
     const int cell = blockIdx.x;
     const long long vb = (long long)cell * V, eb = (long long)cell * E, nv = a.nv;
     double *er = a.scratch + eb * 7;
-    for (int k = tid; k < 6 * V; k += T) snbr[k] = a.nbr[k];
     for (int e = tid; e < E; e += T) {
         double e1[3], e2[3];
         int ia, ib, ic;
@@ -473,94 +480,128 @@ membrane_adjoint_solve_kernel(const MembraneAdjArgs a)
         er[7 * e] = sqrt(g11 * g22 - g12 * g12);
     }
     __syncthreads();
-    float q[VPT][3], rhs[VPT][3], dsb[VPT];
+    // thread tid owns the forward's solve positions tid + m T (membrane.cu), their rows in registers
+    float q[VPT][3], rhs[VPT][3], dsb[VPT], cf[VPT][6];
+    unsigned nb[VPT][3];   // two 16-bit neighbour positions per register
+    int vid[VPT];
 #pragma unroll
     for (int m = 0; m < VPT; m++) {
-        const int i = tid + m * T;
+        const int p = tid + m * T;
         dsb[m] = 0.f;
+        vid[m] = 0;
+#pragma unroll
         for (int c = 0; c < 3; c++) { q[m][c] = 0.f; rhs[m][c] = 0.f; }
-        if (i >= V) continue;
-        double off[6] = {0, 0, 0, 0, 0, 0}, dg = 0.0, s = 0.0;
-        for (int k = __ldg(&a.v2e_off[i]); k < __ldg(&a.v2e_off[i + 1]); k++) {
-            const int pk = __ldg(&a.v2e[k]);
-            const double ga = er[7 * v2e_elem(pk)];
-            dg += ga / 12.0;
-            off[v2e_sa(pk)] += ga / 24.0;
-            off[v2e_sb(pk)] += ga / 24.0;
-            s += ga / 6.0;
+#pragma unroll
+        for (int t = 0; t < 6; t++) cf[m][t] = 0.f;
+#pragma unroll
+        for (int t = 0; t < 3; t++) nb[m][t] = 0u;
+        if (p >= V) continue;
+        const int i = __ldg(&a.vord[p]);
+        vid[m] = i;
+        const int k0 = __ldg(&a.v2e_off[i]), k1 = __ldg(&a.v2e_off[i + 1]);
+        // all incidence entries, then all areas, then the sums (in list order)
+        int pk[6];
+        double ga[6], off[6] = {0, 0, 0, 0, 0, 0}, dg = 0.0, s = 0.0;
+#pragma unroll
+        for (int j = 0; j < 6; j++) pk[j] = k0 + j < k1 ? __ldg(&a.v2e[k0 + j]) : 0;
+#pragma unroll
+        for (int j = 0; j < 6; j++) ga[j] = k0 + j < k1 ? er[7 * v2e_elem(pk[j])] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 6; j++) {
+            if (k0 + j >= k1) break;
+            dg += ga[j] * (1.0 / 12.0);
+            const int sa = v2e_sa(pk[j]), sb = v2e_sb(pk[j]);
+#pragma unroll
+            for (int t = 0; t < 6; t++) off[t] += (t == sa || t == sb) ? ga[j] * (1.0 / 24.0) : 0.0;
+            s += ga[j] * (1.0 / 6.0);
         }
-        for (int t = 0; t < 6; t++) coef[t * V + i] = (float)(off[t] / dg);
+        const double idg = 1.0 / dg, is = 1.0 / s;
+#pragma unroll
+        for (int t = 0; t < 6; t++) {
+            const int j = (int)__ldg(&a.nbrp[t * V + p]);
+            const unsigned id = (unsigned)(j >= 0 ? j : p);   // a missing neighbour: itself with coefficient 0
+            nb[m][t >> 1] |= (t & 1) ? id << 16 : id;
+            cf[m][t] = j >= 0 ? (float)(off[t] * idg) : 0.f;
+        }
         double d = 0.0;
+#pragma unroll
         for (int c = 0; c < 3; c++) {
             const double fv = a.Fv[(long long)c * nv + vb + i], fb = a.Fv_bar[(long long)c * nv + vb + i];
-            const double qc = -fv / s;
+            const double qc = -fv * is;
             q[m][c] = (float)qc;
             d -= qc * fb;
-            rhs[m][c] = (float)(-s * fb / dg);
+            rhs[m][c] = (float)(-s * fb * idg);
         }
         dsb[m] = (float)d;
     }
-    __syncthreads();
     // lambda = M^-1 q_bar: Chebyshev on D^-1 M with the forward's bounds [1/2, 2]
     const float theta = 1.25f, delta = 0.75f, sigma = theta / delta;
     float x[VPT][3], r[VPT][3], dd[VPT][3];
     float rho = 1.0f / sigma;
 #pragma unroll
     for (int m = 0; m < VPT; m++) {
-        const int i = tid + m * T;
-        for (int c = 0; c < 3; c++) { x[m][c] = 0.f; r[m][c] = rhs[m][c]; dd[m][c] = rhs[m][c] / theta; }
-        if (i < V) dbuf[i] = make_float4(dd[m][0], dd[m][1], dd[m][2], 0.f);
+        const int p = tid + m * T;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            x[m][c] = 0.f; r[m][c] = rhs[m][c]; dd[m][c] = rhs[m][c] / theta;
+            if (p < V) dbuf[c * V + p] = dd[m][c];
+        }
     }
     __syncthreads();
     for (int it = 0; it < a.niter; it++) {
-        const float4 *cur = dbuf + (it & 1) * V;
-        float4 *nxt = dbuf + ((it + 1) & 1) * V;
+        const float *cur = dbuf + (it & 1) * 3 * V;
+        float *nxt = dbuf + ((it + 1) & 1) * 3 * V;
         const float rho_n = 1.0f / (2.0f * sigma - rho);
         const float c1 = rho_n * rho, c2 = 2.0f * rho_n / delta;
 #pragma unroll
         for (int m = 0; m < VPT; m++) {
-            const int i = tid + m * T;
-            if (i >= V) continue;
-            float ad0 = dd[m][0], ad1 = dd[m][1], ad2 = dd[m][2];
-            for (int s = 0; s < 6; s++) {
-                const int j = snbr[s * V + i];
-                if (j >= 0) {
-                    const float w = coef[s * V + i];
-                    const float4 dj = cur[j];
-                    ad0 += w * dj.x; ad1 += w * dj.y; ad2 += w * dj.z;
-                }
+            const int p = tid + m * T;
+            if (p >= V) continue;
+            float ad[3] = {dd[m][0], dd[m][1], dd[m][2]};
+#pragma unroll
+            for (int t = 0; t < 6; t++) {
+                const unsigned j = (t & 1) ? nb[m][t >> 1] >> 16 : nb[m][t >> 1] & 0xFFFFu;
+#pragma unroll
+                for (int c = 0; c < 3; c++) ad[c] += cf[m][t] * cur[c * V + j];
             }
-            x[m][0] += dd[m][0]; x[m][1] += dd[m][1]; x[m][2] += dd[m][2];
-            r[m][0] -= ad0; r[m][1] -= ad1; r[m][2] -= ad2;
-            for (int c = 0; c < 3; c++) dd[m][c] = c1 * dd[m][c] + c2 * r[m][c];
-            nxt[i] = make_float4(dd[m][0], dd[m][1], dd[m][2], 0.f);
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                x[m][c] += dd[m][c];
+                r[m][c] -= ad[c];
+                dd[m][c] = c1 * dd[m][c] + c2 * r[m][c];
+                nxt[c * V + p] = dd[m][c];
+            }
         }
         rho = rho_n;
         __syncthreads();
     }
 #pragma unroll
     for (int m = 0; m < VPT; m++) {
-        const int i = tid + m * T;
-        if (i >= V) continue;
-        a.lam[vb + i] = make_float4(x[m][0], x[m][1], x[m][2], 0.f);
-        a.qv[vb + i] = make_float4(q[m][0], q[m][1], q[m][2], 0.f);
-        a.dsb[vb + i] = dsb[m];
+        if (tid + m * T >= V) continue;
+        const long long i = vb + vid[m];
+        a.lam[i] = make_float4(x[m][0], x[m][1], x[m][2], 0.f);
+        a.qv[i] = make_float4(q[m][0], q[m][1], q[m][2], 0.f);
+        a.dsb[i] = dsb[m];
     }
 }
 
 constexpr int MEM_ADJ_ELEM_THREADS = 128;
 
-// One thread per element of any cell: the adjoints of (load on b, load on c,
+// Eight threads per element of any cell: the adjoints of (load on b, load on c,
 // gab) from lambda, q and ds_bar of the element's vertices, contracted with
-// the Jacobian of element_loads (seven dual passes: e1, e2, C).  Writes the
-// edge adjoints to scratch[7 e + 1 .. 6] and adds dL/dC to cbar.
+// the Jacobian of element_loads (seven dual passes: e1, e2, C).  Thread k < 7 of
+// an element runs the pass of input k (one after another in one thread, the
+// passes left a few cells' elements waiting on seven FP64 chains: 8.8 -> 5.8 us
+// for 1280 elements).
+// Writes the edge adjoints to scratch[7 e + 1 .. 6] and adds dL/dC to cbar.
 __global__ void __launch_bounds__(MEM_ADJ_ELEM_THREADS)
 membrane_adjoint_element_kernel(const MembraneAdjArgs a)
 {
     __shared__ double red[MEM_ADJ_ELEM_THREADS / 32];
-    const long long eg = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, eg = t >> 3;
+    const int k = (int)(t & 7);
     double cb = 0.0;
-    if (eg < a.ne) {
+    if (eg < a.ne && k < 7) {
         const int cell = (int)(eg / a.E), e = (int)(eg - (long long)cell * a.E);
         const long long vb = (long long)cell * a.V;
         double e1[3], e2[3];
@@ -577,19 +618,16 @@ membrane_adjoint_element_kernel(const MembraneAdjArgs a)
         const double bCb[3] = {(double)lc.x - la.x, (double)lc.y - la.y, (double)lc.z - la.z};
         const double4 G = a.gref[eg];
         double *er = a.scratch + 7 * eg;
-#pragma unroll 1
-        for (int k = 0; k < 7; k++) {
-            Dual<double> d1[3], d2[3], oB[3], oC[3], og;
-            for (int c = 0; c < 3; c++) {
-                d1[c] = Dual<double>(e1[c], k == c ? 1.0 : 0.0);
-                d2[c] = Dual<double>(e2[c], k == 3 + c ? 1.0 : 0.0);
-            }
-            const Dual<double> Cd(a.C, k == 6 ? 1.0 : 0.0);
-            element_loads<Dual<double>>(d1, d2, G.x, G.y, G.z, G.w, Cd, a.rgs, a.law, oB, oC, og);
-            double s = og.d * gb;
-            for (int c = 0; c < 3; c++) s += oB[c].d * bBb[c] + oC[c].d * bCb[c];
-            if (k < 6) er[1 + k] = s; else cb = s;
+        Dual<double> d1[3], d2[3], oB[3], oC[3], og;
+        for (int c = 0; c < 3; c++) {
+            d1[c] = Dual<double>(e1[c], k == c ? 1.0 : 0.0);
+            d2[c] = Dual<double>(e2[c], k == 3 + c ? 1.0 : 0.0);
         }
+        const Dual<double> Cd(a.C, k == 6 ? 1.0 : 0.0);
+        element_loads<Dual<double>>(d1, d2, G.x, G.y, G.z, G.w, Cd, a.rgs, a.law, oB, oC, og);
+        double s = og.d * gb;
+        for (int c = 0; c < 3; c++) s += oB[c].d * bBb[c] + oC[c].d * bCb[c];
+        if (k < 6) er[1 + k] = s; else cb = s;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) cb += __shfl_xor_sync(0xffffffffu, cb, o);
@@ -611,35 +649,31 @@ __global__ void membrane_adjoint_vertex_kernel(const MembraneAdjArgs a)
     const int cell = (int)(t / a.V), i = (int)(t - (long long)cell * a.V);
     const double *er = a.scratch + 7 * ((long long)cell * a.E);
     double xb[3] = {0.0, 0.0, 0.0};
-    for (int k = __ldg(&a.v2e_off[i]); k < __ldg(&a.v2e_off[i + 1]); k++) {
-        const int pk = __ldg(&a.v2e[k]);
-        const double *rec = er + 7 * v2e_elem(pk);
-        const int en = v2e_en(pk);
+    const int k0 = __ldg(&a.v2e_off[i]), k1 = __ldg(&a.v2e_off[i + 1]);
+    int pk[6];   // at most six elements per vertex (checked when the topology is built): all loads before the sums
+    double ra[6][3], rb[6][3];
+#pragma unroll
+    for (int j = 0; j < 6; j++) pk[j] = k0 + j < k1 ? __ldg(&a.v2e[k0 + j]) : 0;
+#pragma unroll
+    for (int j = 0; j < 6; j++)
+#pragma unroll
         for (int c = 0; c < 3; c++) {
-            if (en == 0) xb[c] -= rec[1 + c] + rec[4 + c];
-            else if (en == 1) xb[c] += rec[1 + c];
-            else xb[c] += rec[4 + c];
+            const double *rec = er + 7 * v2e_elem(pk[j]);
+            ra[j][c] = k0 + j < k1 && v2e_en(pk[j]) != 2 ? rec[1 + c] : 0.0;
+            rb[j][c] = k0 + j < k1 && v2e_en(pk[j]) != 1 ? rec[4 + c] : 0.0;
         }
-    }
+#pragma unroll
+    for (int j = 0; j < 6; j++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            if (k0 + j >= k1) continue;
+            const double r = ra[j][c] + rb[j][c];
+            xb[c] += v2e_en(pk[j]) == 0 ? -r : r;
+        }
     for (int c = 0; c < 3; c++) a.Xd_bar[(long long)c * a.nv + t] = xb[c];
 }
 
 // ---- volume correction, reversed ------------------------------------------
-
-// Normal, area and volume contribution of one triangle as volume.cu's
-// ele_normal computes them, generic in the scalar type.
-template <typename T>
-__device__ __forceinline__ void tri_geom(const T (&pa)[3], const T (&pb)[3], const T (&pc)[3], T (&n)[3], T &dS, T &vt)
-{
-    const T v1x = pb[0] - pa[0], v1y = pb[1] - pa[1], v1z = pb[2] - pa[2];
-    const T v2x = pc[0] - pa[0], v2y = pc[1] - pa[1], v2z = pc[2] - pa[2];
-    const T c0 = v1y * v2z - v1z * v2y, c1 = v1z * v2x - v1x * v2z, c2 = v1x * v2y - v1y * v2x;
-    const T nc = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
-    n[0] = c0 / nc; n[1] = c1 / nc; n[2] = c2 / nc;
-    dS = nc / 2.0;
-    const T rx = (pa[0] + pb[0] + pc[0]) / 3.0, ry = (pa[1] + pb[1] + pc[1]) / 3.0, rz = (pa[2] + pb[2] + pc[2]) / 3.0;
-    vt = (rx * n[0] + ry * n[1] + rz * n[2]) * dS / 3.0;
-}
 
 constexpr int VC_ADJ_THREADS = 1024;
 constexpr double VC_COEFF = 0.1;     // COEFF_VOL_CHANGE (volume_correction.cu:14)
@@ -651,9 +685,17 @@ constexpr double VC_TOL = 1.0e-3;    // percent (volume_correction.cu:15)
 // its elements' unit normals), storing the positions before each move, then
 // reverses the moves: for a move x' = x + s(x) n(x),
 //   x_bar += s (dn/dx)^T x'_bar + (ds/dx)^T (sum_v n_v . x'_bar_v)
-// with ds/dx = -0.3 (dV/dx / A - (V - V0) / A^2 dA/dx); all three are sums
-// over triangles, differentiated per triangle with dual numbers (nine passes).
+// with ds/dx = -0.3 (dV/dx / A - (V - V0) / A^2 dA/dx).  All of it is a sum over
+// triangles.  With c = (B - A) x (C - A), n = c / |c| and W the sum of x'_bar_v /
+// (elements of v) over the triangle's vertices, sum_v n_v . x'_bar_v is the sum of
+// n . W, the adjoint of c is
+//   c_bar = s (W - (n . W) n) / |c| + al (A + B + C) / 18 + be n / 2
+// (al, be the adjoints of the volume and the area: V = sum (A + B + C) . c / 18,
+// A = sum |c| / 2), and those of B - A and C - A are (C - A) x c_bar and
+// c_bar x (B - A); every vertex also takes al c / 18.
 // The final z wrap is a translation.  Writes Xa_bar = (reversed X_bar) + Xd_bar.
+// (Nine forward-mode passes per triangle in place of the closed form, and normals
+// formed per vertex, took 130 us against 51 for one cell of 642 vertices and a few moves.)
 __global__ void __launch_bounds__(VC_ADJ_THREADS, 1)
 volume_adjoint_kernel(const Geom g, const VolumeAdjArgs a)
 {
@@ -664,7 +706,8 @@ volume_adjoint_kernel(const Geom g, const VolumeAdjArgs a)
     const int V = a.V, E = a.E, tid = threadIdx.x, T = blockDim.x, cell = blockIdx.x, N = a.ncell;
     const long long vb = (long long)cell * V, nv = a.nv;
     double *hist = a.hist + (long long)cell * a.kmax * 3 * V;   // positions before each move
-    double *er = a.escr + (long long)cell * E * 9;              // per triangle: adjoints of its 3 vertices
+    // per triangle: its normal in the replay, then the adjoints of its 3 vertices (written and read by this block)
+    double *er = a.escr + (long long)cell * E * 9;
     const double gz = a.gx[2 * N + cell];
     for (int v = tid; v < V; v += T) {
         p[v] = a.Xa[vb + v];
@@ -676,92 +719,105 @@ volume_adjoint_kernel(const Geom g, const VolumeAdjArgs a)
         for (int c = 0; c < 3; c++) pb[c * V + v] = a.X_bar[(long long)c * nv + vb + v];
     }
     __syncthreads();
-    auto tri_at = [&](const double *P, int e, double (&A)[3], double (&B)[3], double (&Cc)[3]) {
-        const int ia = __ldg(&a.tri[3 * e]), ib = __ldg(&a.tri[3 * e + 1]), ic = __ldg(&a.tri[3 * e + 2]);
-        for (int c = 0; c < 3; c++) { A[c] = P[c * V + ia]; B[c] = P[c * V + ib]; Cc[c] = P[c * V + ic]; }
+    auto tri_at = [&](int e, int (&id)[3], double (&A)[3], double (&B)[3], double (&C)[3]) {
+        for (int t = 0; t < 3; t++) id[t] = __ldg(&a.tri[3 * e + t]);
+        for (int c = 0; c < 3; c++) { A[c] = p[c * V + id[0]]; B[c] = p[c * V + id[1]]; C[c] = p[c * V + id[2]]; }
     };
-    auto vol_area = [&](const double *P, double &vol, double &area) {   // as volume.cu measures them
+    auto cross = [](const double (&u)[3], const double (&w)[3], double (&r)[3]) {
+        r[0] = u[1] * w[2] - u[2] * w[1]; r[1] = u[2] * w[0] - u[0] * w[2]; r[2] = u[0] * w[1] - u[1] * w[0];
+    };
+    // volume and area as volume.cu measures them
+    auto vol_area = [&](double &vol, double &area) {
         double sv = 0.0, sa = 0.0;
         for (int e = tid; e < E; e += T) {
-            double A[3], B[3], Cc[3];
-            tri_at(P, e, A, B, Cc);
-            tri_measure(A, B, Cc, sv, sa);
+            int id[3];
+            double A[3], B[3], C[3];
+            tri_at(e, id, A, B, C);
+            tri_measure(A, B, C, sv, sa);
         }
         vol = block_sum_r(sv, red) / 18.0;
         area = block_sum_r(sa, red) / 2.0;
-    };
-    auto mean_normal = [&](const double *P, int v, double (&nn)[3]) {
-        const int k0 = __ldg(&a.v2e_off[v]), k1 = __ldg(&a.v2e_off[v + 1]), nne = k1 - k0;
-        nn[0] = nn[1] = nn[2] = 0.0;
-        for (int k = k0; k < k1; k++) {
-            double A[3], B[3], Cc[3], n[3], dS, vt;
-            tri_at(P, v2e_elem(__ldg(&a.v2e[k])), A, B, Cc);
-            tri_geom<double>(A, B, Cc, n, dS, vt);
-            for (int c = 0; c < 3; c++) nn[c] += n[c] / nne;
-        }
     };
     // forward replay
     const double V0 = a.vol0[cell];
     int moves = 0;
     for (int it = 1;; it++) {
         double vol, area;
-        vol_area(p, vol, area);
+        vol_area(vol, area);
         if (fabs(vol - V0) / V0 * 100.0 < VC_TOL) break;
         if (moves >= a.kmax || it >= 1000) {   // more moves than the history holds: reverse only those recorded
             if (tid == 0) atomicOr(a.status, 1);
             break;
         }
+        for (int e = tid; e < E; e += T) {
+            int id[3];
+            double A[3], B[3], C[3], v1[3], v2[3], cr[3];
+            tri_at(e, id, A, B, C);
+            for (int c = 0; c < 3; c++) { v1[c] = B[c] - A[c]; v2[c] = C[c] - A[c]; }
+            cross(v1, v2, cr);
+            const double inv = 1.0 / sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
+            for (int c = 0; c < 3; c++) er[9 * e + c] = cr[c] * inv;
+        }
         for (int k = tid; k < 3 * V; k += T) hist[(long long)moves * 3 * V + k] = p[k];
         const double s = -18.0 * (vol - V0) / area / 6.0 * VC_COEFF;
-        double disp[4][3];
-        for (int m = 0; m < 4; m++) {
-            const int v = tid + m * T;
-            if (v >= V) continue;
-            double nn[3];
-            mean_normal(p, v, nn);
-            for (int c = 0; c < 3; c++) disp[m][c] = s * nn[c];
-        }
         __syncthreads();
-        for (int m = 0; m < 4; m++) {
-            const int v = tid + m * T;
-            if (v >= V) continue;
-            for (int c = 0; c < 3; c++) p[c * V + v] += disp[m][c];
+        for (int v = tid; v < V; v += T) {
+            const int k0 = __ldg(&a.v2e_off[v]), k1 = __ldg(&a.v2e_off[v + 1]);
+            double nn[3] = {0.0, 0.0, 0.0};
+            for (int k = k0; k < k1; k++) {
+                const double *n = er + 9 * v2e_elem(__ldg(&a.v2e[k]));
+                for (int c = 0; c < 3; c++) nn[c] += n[c];
+            }
+            const double m = s / (double)(k1 - k0);
+            for (int c = 0; c < 3; c++) p[c * V + v] += m * nn[c];
         }
         __syncthreads();
         moves++;
     }
     // reverse the moves
     for (int j = moves - 1; j >= 0; j--) {
-        const double *P = hist + (long long)j * 3 * V;
-        double vol, area;
-        vol_area(P, vol, area);
-        const double s = -18.0 * (vol - V0) / area / 6.0 * VC_COEFF;
-        double w = 0.0;
-        for (int v = tid; v < V; v += T) {
-            double nn[3];
-            mean_normal(P, v, nn);
-            w += nn[0] * pb[v] + nn[1] * pb[V + v] + nn[2] * pb[2 * V + v];
+        for (int k = tid; k < 3 * V; k += T) p[k] = hist[(long long)j * 3 * V + k];
+        __syncthreads();
+        auto weight = [&](const int (&id)[3], double (&W)[3]) {
+            W[0] = W[1] = W[2] = 0.0;
+            for (int t = 0; t < 3; t++) {
+                const double inv = 1.0 / (double)(__ldg(&a.v2e_off[id[t] + 1]) - __ldg(&a.v2e_off[id[t]]));
+                for (int c = 0; c < 3; c++) W[c] += pb[c * V + id[t]] * inv;
+            }
+        };
+        double sv = 0.0, sa = 0.0, sw = 0.0;
+        for (int e = tid; e < E; e += T) {
+            int id[3];
+            double A[3], B[3], C[3], v1[3], v2[3], cr[3], W[3];
+            tri_at(e, id, A, B, C);
+            tri_measure(A, B, C, sv, sa);
+            weight(id, W);
+            for (int c = 0; c < 3; c++) { v1[c] = B[c] - A[c]; v2[c] = C[c] - A[c]; }
+            cross(v1, v2, cr);
+            sw += (cr[0] * W[0] + cr[1] * W[1] + cr[2] * W[2]) / sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
         }
-        w = block_sum_r(w, red);
+        const double vol = block_sum_r(sv, red) / 18.0, area = block_sum_r(sa, red) / 2.0, w = block_sum_r(sw, red);
+        const double s = -18.0 * (vol - V0) / area / 6.0 * VC_COEFF;
         const double al = -0.3 * w / area, be = 0.3 * w * (vol - V0) / (area * area);
         for (int e = tid; e < E; e += T) {
-            const int id[3] = {__ldg(&a.tri[3 * e]), __ldg(&a.tri[3 * e + 1]), __ldg(&a.tri[3 * e + 2])};
-            double W[3] = {0.0, 0.0, 0.0}, x0[3][3];
-            for (int t = 0; t < 3; t++) {
-                const int u = id[t];
-                const double inv = 1.0 / (double)(__ldg(&a.v2e_off[u + 1]) - __ldg(&a.v2e_off[u]));
-                for (int c = 0; c < 3; c++) { W[c] += pb[c * V + u] * inv; x0[t][c] = P[c * V + u]; }
-            }
-#pragma unroll 1
-            for (int k = 0; k < 9; k++) {
-                Dual<double> A[3], B[3], Cc[3], n[3], dS, vt;
-                for (int c = 0; c < 3; c++) {
-                    A[c] = Dual<double>(x0[0][c], k == c ? 1.0 : 0.0);
-                    B[c] = Dual<double>(x0[1][c], k == 3 + c ? 1.0 : 0.0);
-                    Cc[c] = Dual<double>(x0[2][c], k == 6 + c ? 1.0 : 0.0);
-                }
-                tri_geom<Dual<double>>(A, B, Cc, n, dS, vt);
-                er[9 * e + k] = s * (n[0].d * W[0] + n[1].d * W[1] + n[2].d * W[2]) + al * vt.d + be * dS.d;
+            int id[3];
+            double A[3], B[3], C[3], v1[3], v2[3], cr[3], W[3], cb[3], b1[3], b2[3];
+            tri_at(e, id, A, B, C);
+            weight(id, W);
+            for (int c = 0; c < 3; c++) { v1[c] = B[c] - A[c]; v2[c] = C[c] - A[c]; }
+            cross(v1, v2, cr);
+            const double inv = 1.0 / sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
+            double n[3], nW = 0.0;
+            for (int c = 0; c < 3; c++) { n[c] = cr[c] * inv; nW += n[c] * W[c]; }
+            for (int c = 0; c < 3; c++)
+                cb[c] = s * inv * (W[c] - nW * n[c]) + al / 18.0 * (A[c] + B[c] + C[c]) + 0.5 * be * n[c];
+            cross(v2, cb, b1);
+            cross(cb, v1, b2);
+            for (int c = 0; c < 3; c++) {
+                const double all = al / 18.0 * cr[c];
+                er[9 * e + c] = all - b1[c] - b2[c];
+                er[9 * e + 3 + c] = all + b1[c];
+                er[9 * e + 6 + c] = all + b2[c];
             }
         }
         __syncthreads();
@@ -825,16 +881,15 @@ cudaError_t adjoint_setup(int optin)
 void launch_membrane_adjoint(const MembraneAdjArgs &a, cudaStream_t s)
 {
     if (a.ncell <= 0) return;
-    const int vpt = (a.V + MEM_ADJ_THREADS - 1) / MEM_ADJ_THREADS;
-    const int T = (((a.V + vpt - 1) / vpt) + 31) / 32 * 32;
-    const size_t smem = (size_t)membrane_smem_bytes(a.V);
+    const int vpt = membrane_default_vpt(a.V), T = membrane_threads(a.V, vpt);
+    const size_t smem = 24 * (size_t)a.V;   // the solve's two buffers
     switch (vpt) {
     case 1: membrane_adjoint_solve_kernel<1><<<a.ncell, T, smem, s>>>(a); break;
     case 2: membrane_adjoint_solve_kernel<2><<<a.ncell, T, smem, s>>>(a); break;
     case 3: membrane_adjoint_solve_kernel<3><<<a.ncell, T, smem, s>>>(a); break;
     default: membrane_adjoint_solve_kernel<4><<<a.ncell, T, smem, s>>>(a); break;
     }
-    membrane_adjoint_element_kernel<<<(unsigned)((a.ne + MEM_ADJ_ELEM_THREADS - 1) / MEM_ADJ_ELEM_THREADS),
+    membrane_adjoint_element_kernel<<<(unsigned)((8 * a.ne + MEM_ADJ_ELEM_THREADS - 1) / MEM_ADJ_ELEM_THREADS),
                                       MEM_ADJ_ELEM_THREADS, 0, s>>>(a);
     membrane_adjoint_vertex_kernel<<<(unsigned)((a.nv + 127) / 128), 128, 0, s>>>(a);
 }
@@ -842,7 +897,7 @@ void launch_membrane_adjoint(const MembraneAdjArgs &a, cudaStream_t s)
 void launch_volume_adjoint(const Geom &g, const VolumeAdjArgs &a, cudaStream_t s)
 {
     if (a.ncell <= 0) return;
-    volume_adjoint_kernel<<<a.ncell, VC_ADJ_THREADS, volume_adjoint_smem_bytes(a.V), s>>>(g, a);
+    volume_adjoint_kernel<<<a.ncell, volume_threads(a.V), volume_adjoint_smem_bytes(a.V), s>>>(g, a);
 }
 
 }  // namespace rbc

@@ -57,10 +57,10 @@ namespace rbc {
 
 constexpr int MEM_MAX_THREADS = 1024;
 
-// pos 24V (then the solve's two d-buffers, 3 x V floats each), coef 24V, and 12V that the adjoint's
-// membrane pass uses for its neighbour table (this kernel reads its neighbours
-// from global memory once, into registers)
-int membrane_smem_bytes(int V) { return 68 * V; }
+// pos 24V (then the solve's two d-buffers, 3 x V floats each), 8V unused, coef 24V
+int membrane_smem_bytes(int V) { return 56 * V; }
+// what the vertices per cell are limited by
+int membrane_limit_bytes(int V) { return 68 * V; }
 
 __device__ __forceinline__ double mimage(double d, double L) {
     if (d > L * 0.5) d -= L; else if (d < -L * 0.5) d += L;

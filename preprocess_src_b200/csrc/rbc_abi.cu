@@ -49,7 +49,6 @@ struct CellGroup {
     void *erec = nullptr;   // membrane element records, [ne][3] 4-vectors of float or double
     float *U = nullptr, *Fv = nullptr;
     int *tri = nullptr, *v2e_off = nullptr, *v2e = nullptr;
-    int16_t *nbr = nullptr;
     int16_t *nbrp = nullptr;  // neighbours by solve position ([6][V]) and the vertex at each position ([V])
     int *vord = nullptr;
     int4 *visit = nullptr;   // bending visits [E][3], allocated when BR != 0
@@ -76,7 +75,6 @@ struct rbc_handle {
     double4 *&gref = cg[0].gref;
     float *&U = cg[0].U, *&Fv = cg[0].Fv;
     int *&tri = cg[0].tri, *&v2e_off = cg[0].v2e_off, *&v2e = cg[0].v2e;
-    int16_t *&nbr = cg[0].nbr;
     double *&vol0 = cg[0].vol0, *&gx = cg[0].gx;
     long long nref_nodes = 0;
     cudaStream_t stream = nullptr;
@@ -259,7 +257,7 @@ WallVel wall_velocities(const rbc_handle *h, int step)
 // reference's link-count check, and the packed incidence entries used by the
 // membrane and volume kernels.
 int build_topology(rbc_handle *h, const CellGroup &c, const int *tri, std::vector<int> &off, std::vector<int> &packed,
-                   std::vector<int16_t> &nbr6, std::vector<int16_t> &nbrp6, std::vector<int> &vord)
+                   std::vector<int16_t> &nbrp6, std::vector<int> &vord)
 {
     const int V = c.V, E = c.E;
     std::vector<std::vector<int>> nl(V), el(V);
@@ -315,10 +313,8 @@ int build_topology(rbc_handle *h, const CellGroup &c, const int *tri, std::vecto
     }
     off.assign(V + 1, 0);
     packed.clear();
-    nbr6.assign((size_t)6 * V, (int16_t)-1);
     for (int i = 0; i < V; i++) {
         off[i] = (int)packed.size();
-        for (size_t s = 0; s < nl[i].size(); s++) nbr6[s * V + i] = (int16_t)nl[i][s];
         for (int e : el[i]) {
             int en = (tri[3 * e] == i) ? 0 : (tri[3 * e + 1] == i ? 1 : 2);
             const int o1 = tri[3 * e + (en + 1) % 3], o2 = tri[3 * e + (en + 2) % 3];
@@ -663,7 +659,7 @@ int build_mask(const rbc_params *p, const int *bc, std::vector<uint32_t> &mask)
 
 void free_group(CellGroup &c)
 {
-    void *cp[] = {c.X, c.Xd, c.gref, c.erec, c.U, c.Fv, c.tri, c.v2e_off, c.v2e, c.nbr, c.nbrp, c.vord, c.visit, c.cs0, c.patch_off,
+    void *cp[] = {c.X, c.Xd, c.gref, c.erec, c.U, c.Fv, c.tri, c.v2e_off, c.v2e, c.nbrp, c.vord, c.visit, c.cs0, c.patch_off,
                   c.patch_vtx, c.patch_stride, c.vol0, c.gx, c.vol_out, c.area_out, c.cen_out, c.qi_acc, c.tp_acc,
                   c.vf, c.bend_rec};
     for (void *q : cp) if (q) cudaFree(q);
@@ -710,7 +706,7 @@ int launch_membrane_range(rbc_handle *h, CellGroup &g, int c0, int c1, cudaStrea
     MembraneArgs a{};
     a.Xd = g.Xd + (size_t)c0 * g.V; a.nv = g.nv; a.ne = g.ne; a.gref = g.gref + (size_t)c0 * g.E;
     a.erec = (char *)g.erec + (size_t)c0 * g.E * rec_bytes;
-    a.tri = g.tri; a.v2e_off = g.v2e_off; a.v2e = g.v2e; a.nbr = g.nbr; a.nbrp = g.nbrp; a.vord = g.vord; a.Fv = g.Fv + (size_t)c0 * g.V;
+    a.tri = g.tri; a.v2e_off = g.v2e_off; a.v2e = g.v2e; a.nbrp = g.nbrp; a.vord = g.vord; a.Fv = g.Fv + (size_t)c0 * g.V;
     a.V = g.V; a.E = g.E; a.ncell = c1 - c0;
     a.C = h->p.C; a.rgs = g.rgs; a.law = h->p.law; a.LX = h->p.LX; a.LZ = h->p.LZ;
     a.niter = h->p.solver_iters > 0 ? h->p.solver_iters : DEFAULT_SOLVER_ITERS;
@@ -753,7 +749,7 @@ MembraneArgs membrane_args(rbc_handle *h, CellGroup &g)
 {
     MembraneArgs a{};
     a.Xd = g.Xd; a.nv = g.nv; a.ne = g.ne; a.gref = g.gref; a.erec = g.erec;
-    a.tri = g.tri; a.v2e_off = g.v2e_off; a.v2e = g.v2e; a.nbr = g.nbr; a.nbrp = g.nbrp; a.vord = g.vord; a.Fv = g.Fv;
+    a.tri = g.tri; a.v2e_off = g.v2e_off; a.v2e = g.v2e; a.nbrp = g.nbrp; a.vord = g.vord; a.Fv = g.Fv;
     a.V = g.V; a.E = g.E; a.ncell = g.ncell;
     a.C = h->p.C; a.rgs = g.rgs; a.law = h->p.law; a.LX = h->p.LX; a.LZ = h->p.LZ;
     a.niter = h->p.solver_iters > 0 ? h->p.solver_iters : DEFAULT_SOLVER_ITERS;
@@ -1344,7 +1340,7 @@ int batch_build(rbc_batch *b)
 // centroids, bending visits.
 struct GroupPrep {
     std::vector<int> off, packed;
-    std::vector<int16_t> nbr6, nbrp6;
+    std::vector<int16_t> nbrp6;
     std::vector<int> vord;
     std::vector<double> vol0, gx, xs;
     std::vector<double4> gref;
@@ -1356,7 +1352,7 @@ int prepare_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, GroupPrep &
 {
     c.ncell = mesh->ncell; c.V = mesh->vertex; c.E = mesh->element;
     c.nv = (long long)c.ncell * c.V; c.ne = (long long)c.ncell * c.E;
-    int rc = build_topology(h, c, mesh->tri, pp.off, pp.packed, pp.nbr6, pp.nbrp6, pp.vord);
+    int rc = build_topology(h, c, mesh->tri, pp.off, pp.packed, pp.nbrp6, pp.vord);
     if (rc) return rc;
     reference_metric(c, mesh->tri, mesh->xr, pp.gref);
     initial_volume(h, c, mesh->tri, mesh->xr, pp.vol0, pp.gx);
@@ -1380,7 +1376,7 @@ int upload_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, const GroupP
     CK(cudaMalloc(&c.erec, (size_t)c.ne * 12 * (h->p.membrane_fp64 ? sizeof(double) : sizeof(float))));
     TRYG(dalloc(h, &c.U, 3 * c.nv)); TRYG(dalloc(h, &c.Fv, 3 * c.nv));
     TRYG(dalloc(h, &c.tri, 3 * c.E)); TRYG(dalloc(h, &c.v2e_off, c.V + 1)); TRYG(dalloc(h, &c.v2e, pp.packed.size()));
-    TRYG(dalloc(h, &c.nbr, 6 * c.V)); TRYG(dalloc(h, &c.nbrp, 6 * c.V)); TRYG(dalloc(h, &c.vord, c.V));
+    TRYG(dalloc(h, &c.nbrp, 6 * c.V)); TRYG(dalloc(h, &c.vord, c.V));
     if (!pp.visit.empty()) {
         TRYG(dalloc(h, &c.visit, pp.visit.size()));
         CK(cudaMemcpy(c.visit, pp.visit.data(), sizeof(int4) * pp.visit.size(), cudaMemcpyHostToDevice));
@@ -1403,7 +1399,6 @@ int upload_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, const GroupP
     CK(cudaMemcpy(c.tri, mesh->tri, 4 * 3 * c.E, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.v2e_off, pp.off.data(), 4 * (c.V + 1), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.v2e, pp.packed.data(), 4 * pp.packed.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c.nbr, pp.nbr6.data(), 2 * 6 * c.V, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.nbrp, pp.nbrp6.data(), 2 * 6 * c.V, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.vord, pp.vord.data(), 4 * c.V, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.patch_off, poff.data(), 4 * poff.size(), cudaMemcpyHostToDevice));
@@ -1504,7 +1499,7 @@ int rbc_create(const rbc_params *p, const rbc_mesh *mesh, const int *bc, rbc_han
     if (cells) {
         if (mesh->vertex < 4 || mesh->element < 4 || !mesh->tri || !mesh->xr)
             return fail(nullptr, RBC_ERR_ARG, "mesh needs vertex, element >= 4, tri and xr");
-        if (membrane_smem_bytes(mesh->vertex) > 227 * 1024 || mesh->vertex > 4096)
+        if (membrane_limit_bytes(mesh->vertex) > 227 * 1024 || mesh->vertex > 4096)
             return fail(nullptr, RBC_ERR_UNSUPPORTED, "more vertices per cell than one CTA holds (max 3874)");
         if (mesh->element >= (1 << 24)) return fail(nullptr, RBC_ERR_UNSUPPORTED, "too many elements per cell");
     }
@@ -1555,7 +1550,7 @@ int rbc_create(const rbc_params *p, const rbc_mesh *mesh, const int *bc, rbc_han
         if (!e) e = (int)lattice_io_setup();
         if (!e) e = (int)cell_io_setup();
         if (e) { h->err = std::string("kernel attributes: ") + cudaGetErrorString((cudaError_t)e); return bail(RBC_ERR_CUDA); }
-        if (cells && membrane_smem_bytes(mesh->vertex) > mem_max) {
+        if (cells && membrane_limit_bytes(mesh->vertex) > mem_max) {
             h->err = "more vertices per cell than one CTA's shared memory holds";
             return bail(RBC_ERR_UNSUPPORTED);
         }
@@ -2642,7 +2637,7 @@ int adjoint_reserve(rbc_handle *h, int K, int nseg)
     TRYA(adj_alloc(h, &a->ck_itd, nck));
     TRYA(adj_alloc(h, &a->sg, S * nq)); TRYA(adj_alloc(h, &a->sF, S * 3 * n)); TRYA(adj_alloc(h, &a->sFv, S * nv3));
     TRYA(adj_alloc(h, &a->suvr, S * n)); TRYA(adj_alloc(h, &a->sdrv, S)); TRYA(adj_alloc(h, &a->sfac, S));
-    TRYA(adj_alloc(h, &a->sX, S * nv3)); TRYA(adj_alloc(h, &a->sXd, S * nv3)); TRYA(adj_alloc(h, &a->sXa, S * nv3));
+    TRYA(adj_alloc(h, &a->sX, S * nv3)); TRYA(adj_alloc(h, &a->sXd, 2 * nv3)); TRYA(adj_alloc(h, &a->sXa, S * nv3));
     TRYA(adj_alloc(h, &a->sgx, S * N3));
     TRYA(adj_alloc(h, &a->gbar[0], nq)); TRYA(adj_alloc(h, &a->gbar[1], nq));
     TRYA(adj_alloc(h, &a->lam, h->nv)); TRYA(adj_alloc(h, &a->qv, h->nv)); TRYA(adj_alloc(h, &a->dsb, h->nv));
@@ -2717,9 +2712,15 @@ int adjoint_enqueue_recompute_body(rbc_handle *h, int b, int len)
     int rc;
     for (int t = 0; t < len; t++) {
         const size_t k = (size_t)b * a->K + t;
-        if ((rc = d2d(h, a->sg + k * nq, h->g[h->cur], 4 * nq))) return rc;
+        // the stages work in the store itself: the populations of step t + 1, the forces, the
+        // velocity and the advected positions (fem->xd of step t + 1) are written where the
+        // reversal reads them, the last step's populations and positions to the handle
+        double *const Xa = a->sXa + k * nv3;
+        if (t == 0) {
+            if ((rc = d2d(h, a->sg + k * nq, h->g[h->cur], 4 * nq))) return rc;
+            if ((rc = d2d(h, a->sXd + b * nv3, h->Xd, 8 * nv3))) return rc;
+        }
         if ((rc = d2d(h, a->sX + k * nv3, h->X, 8 * nv3))) return rc;
-        if ((rc = d2d(h, a->sXd + k * nv3, h->Xd, 8 * nv3))) return rc;
         if ((rc = d2d(h, a->sgx + k * N3, h->gx, 8 * N3))) return rc;
         StepBeginArgs sb = step_begin_args(h);
         sb.drive_rec = a->sdrv + k;
@@ -2727,16 +2728,40 @@ int adjoint_enqueue_recompute_body(rbc_handle *h, int b, int len)
         launch_step_begin(sb, h->stream);
         h->launches++;
         CK_LAUNCH();
-        if ((rc = launch_stress(h))) return rc;
-        if ((rc = d2d(h, a->sFv + k * nv3, h->Fv, 4 * nv3))) return rc;
-        if ((rc = launch_spread_stage(h))) return rc;
+        CellGroup &g = h->cg[0];
+        if (h->ncell > 0) {
+            MembraneArgs m = membrane_args(h, g);
+            m.Xd = t == 0 ? h->Xd : Xa - nv3;
+            m.Fv = a->sFv + k * nv3;
+            launch_membrane(m, h->p.membrane_fp64 != 0, h->stream);
+            CK_LAUNCH();
+            SpreadArgs s = spread_args(h, g);
+            s.Fv = m.Fv;
+            launch_spread(h->geo, s, h->stream);
+            h->launches += 2;
+            CK_LAUNCH();
+        }
         launch_force_to_f32(h->geo, h->Fint, a->sF + k * 3 * n, h->stream);   // the force the collision reads
         h->launches++;
         CK_LAUNCH();
-        if ((rc = launch_lbm_stage(h))) return rc;
-        if ((rc = d2d(h, a->suvr + k * n, h->uvr, 16 * n))) return rc;
-        if ((rc = launch_advect_stage(h))) return rc;
-        if ((rc = d2d(h, a->sXa + k * nv3, h->Xd, 8 * nv3))) return rc;
+        LbmArgs l = lbm_args(h, h->cur);
+        l.gin = a->sg + k * nq;
+        if (t + 1 < len) l.gout = a->sg + (k + 1) * nq;
+        l.uvr = a->suvr + k * n;
+        launch_lbm(h->geo, h->p.storage, l, h->stream);
+        h->launches++;
+        CK_LAUNCH();
+        h->cur ^= 1;
+        if ((rc = launch_force_reset_stage(h, h->stream))) return rc;
+        if (h->ncell > 0) {
+            AdvectArgs v = advect_args(h, g);
+            v.Xd = Xa;
+            v.uvr = l.uvr;
+            launch_advect(h->geo, v, h->stream);
+            h->launches++;
+            CK_LAUNCH();
+            if (t + 1 == len && (rc = d2d(h, h->Xd, Xa, 8 * nv3))) return rc;
+        }
         if ((rc = launch_volume_stage(h, h->stream))) return rc;
     }
     return RBC_OK;
@@ -2787,8 +2812,8 @@ int adjoint_enqueue_reverse(rbc_handle *h, int b, int len, int gb)
             h->launches++;
             CK_LAUNCH();
             MembraneAdjArgs ma{};
-            ma.Xd = a->sXd + k * nv3; ma.nv = h->nv; ma.ne = h->ne; ma.gref = h->gref;
-            ma.tri = h->tri; ma.v2e_off = h->v2e_off; ma.v2e = h->v2e; ma.nbr = h->nbr;
+            ma.Xd = t == 0 ? a->sXd + b * nv3 : a->sXa + (k - 1) * nv3; ma.nv = h->nv; ma.ne = h->ne; ma.gref = h->gref;
+            ma.tri = h->tri; ma.v2e_off = h->v2e_off; ma.v2e = h->v2e; ma.nbrp = h->cg[0].nbrp; ma.vord = h->cg[0].vord;
             ma.Fv = a->sFv + k * nv3; ma.Fv_bar = a->Fvbar; ma.Xd_bar = a->Xdbar; ma.scratch = a->mscr;
             ma.lam = a->lam; ma.qv = a->qv; ma.dsb = a->dsb;
             ma.cbar = a->pbar + 2;
@@ -3348,7 +3373,7 @@ int rbc_add_wbc(rbc_handle *h, const rbc_mesh *mesh, double rgs, double br)
     if (h->ngroups > 1) return fail(h, RBC_ERR_STATE, "the white cells are already set");
     if (mesh->vertex < 4 || mesh->element < 4 || !mesh->tri || !mesh->xr)
         return fail(h, RBC_ERR_ARG, "mesh needs vertex, element >= 4, tri and xr");
-    if (membrane_smem_bytes(mesh->vertex) > 227 * 1024 || mesh->vertex > 4096)
+    if (membrane_limit_bytes(mesh->vertex) > 227 * 1024 || mesh->vertex > 4096)
         return fail(h, RBC_ERR_UNSUPPORTED, "more vertices per cell than one CTA holds (max 3874)");
     if (mesh->element >= (1 << 24)) return fail(h, RBC_ERR_UNSUPPORTED, "too many elements per cell");
     if (!(rgs > 0.0) || !std::isfinite(rgs) || !std::isfinite(br)) return fail(h, RBC_ERR_ARG, "rgs must be > 0 and br finite");

@@ -280,8 +280,7 @@ struct MembraneArgs {
     const double4 *gref;      // [ne] reference covariant metric (G11, G12, G22, 1 / det G)
     void *erec;               // [ne][3] element records (Real 4-vectors): scratch written and read by each CTA
     const int *tri, *v2e_off, *v2e;
-    const int16_t *nbr;       // [6][V] local neighbour ids, -1 = none
-    const int16_t *nbrp;      // [6][V] the same neighbours as positions in the solve order, by position
+    const int16_t *nbrp;      // [6][V] neighbours as positions in the solve order, by position; -1 = none
     const int *vord;          // [V] solve order: the vertex at each position
     float *Fv;
     int V, E, ncell;
@@ -292,6 +291,7 @@ struct MembraneArgs {
     int priority;             // launch priority (cudaLaunchAttributePriority)
 };
 int  membrane_smem_bytes(int V);
+int  membrane_limit_bytes(int V);   // bytes per block that bound the vertices per cell
 
 // host helpers of the reference-format files (rbc_abi.cu)
 int reference_mn(int V);
@@ -363,6 +363,7 @@ struct VolumeArgs {
     int cache_normals;        // the block's shared memory holds the cell's unit normals (volume_caches_normals)
 };
 bool volume_caches_normals(int V);
+int volume_threads(int V);   // of a volume correction block
 int  volume_smem_bytes(int V);
 void launch_volume(const Geom &g, const VolumeArgs &a, cudaStream_t s);
 
@@ -434,7 +435,8 @@ struct MembraneAdjArgs {
     const double *Xd; long long nv, ne;
     const double4 *gref;
     const int *tri, *v2e_off, *v2e;
-    const int16_t *nbr;
+    const int16_t *nbrp;       // neighbours by solve position and the vertex at each position (MembraneArgs)
+    const int *vord;
     const float *Fv;           // the step's membrane forces
     const double *Fv_bar;      // their adjoint, [3][nv]
     double *Xd_bar;            // out, [3][nv]

@@ -19,7 +19,7 @@ namespace rbc {
 // threads of a block: one vertex (two elements) each for cells of up to 1024
 // vertices, so small cells meet fewer warps at each barrier and reduction
 constexpr int VOL_THREADS = 1024;
-static int volume_threads(int V) { return V >= VOL_THREADS ? VOL_THREADS : (V + 31) / 32 * 32; }
+int volume_threads(int V) { return V >= VOL_THREADS ? VOL_THREADS : (V + 31) / 32 * 32; }
 constexpr double COEFF_VOL_CHANGE = 0.1;   // volume_correction.cu:14
 constexpr double VC_EPS = 1.0e-3;          // volume_correction.cu:15, percent
 constexpr int VC_ITRMAX = 1000;            // volume_correction.cu:487
