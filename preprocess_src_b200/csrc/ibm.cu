@@ -344,15 +344,23 @@ void launch_spread(const Geom &g, const SpreadArgs &a, cudaStream_t s)
 
 // ---- interpolation + RK4 advection ---------------------------------------
 
-// Four lanes per vertex: lane c of the group owns stencil plane c (16 nodes).
-// The stage-1 stencil is loaded once into registers (u, v, w of 16 nodes) and
-// reused by the later RK stages, whose positions move by u dt / 2 ~ 1e-3 and
+// LANES (2 or 4) lanes per vertex: lane c of the group owns 4 / LANES planes of
+// the stencil (16 nodes each).  The stage-1 stencil is loaded once into registers
+// and reused by the later RK stages, whose positions move by u dt / 2 ~ 1e-3 and
 // almost never leave the stage-1 lattice cell; a stage that does re-gathers.
-// The group sums its partial velocities with two butterfly shuffles.  Stage 1
+// The group sums its partial velocities with butterfly shuffles.  Stage 1
 // locates the vertex in FP64 (positions ~100 lattice units); the later stages'
 // fractions are the stage-1 fraction plus the move u h / dx in FP32 (one more
 // FP32 rounding of a number below 1, where the FP64 position would round the
 // same move to about 1e-14).
+// Two lanes do a third fewer instructions per vertex (each lane evaluates the delta
+// weights itself) and hold twice the stencil: 168 registers, three blocks of 128
+// threads per multiprocessor against two of 256 threads.  That is the better trade
+// where blocks queue, four lanes where a block's own latency is the kernel's time:
+// 200 cells of 2562 vertices 118 -> 106 us, 20 of them 19.3 -> 17.4, one cell of 642
+// 10.5 -> 12.2.  Every product and sum over planes is written with its rounding, so
+// both give the same bits.
+constexpr int ADVECT_VERTICES = 64;   // per pass of a block
 struct Plane16 {
     float u[16], v[16], w[16];
 };
@@ -379,38 +387,33 @@ __device__ __forceinline__ void gather_plane(const Geom &g, const float4 *__rest
     }
 }
 
-__device__ __forceinline__ void lattice_cell(const Geom &g, double px, double py, double pz, int &ix0, int &iy0,
-                                             int &iz0, float &fx, float &fy, float &fz)
+// sum over the lane's planes of wz wy wx value, rows first (63 operations per plane
+// in chains of nine; the product weights wx wy wz would take 68 in chains of 16),
+// then over the vertex's lanes
+template <int LANES>
+__device__ __forceinline__ void contract(const Plane16 (&P)[4 / LANES], const float wx[4], const float wy[4],
+                                         const float (&wz)[4 / LANES], float (&s)[3])
 {
-    const double lx = lat_x(g, px), ly = lat_y(g, py), lz = lat_z(g, pz);
-    const double flx = floor(lx), fly = floor(ly), flz = floor(lz);
-    ix0 = (int)flx - 1; iy0 = (int)fly - 1; iz0 = (int)flz - 1;
-    fx = (float)(lx - flx); fy = (float)(ly - fly); fz = (float)(lz - flz);
-}
-
-__device__ __forceinline__ void contract(const Plane16 &P, const float wx[4], const float wy[4], float wzc,
-                                         float &ur, float &vr, float &wr)
-{
-    float su = 0.f, sv = 0.f, sw = 0.f;
 #pragma unroll
-    for (int b = 0; b < 4; b++) {
-        const float wyz = wy[b] * wzc;
+    for (int k = 0; k < 4 / LANES; k++) {
+        const float *comp[3] = {P[k].u, P[k].v, P[k].w};
 #pragma unroll
-        for (int a = 0; a < 4; a++) {
-            const float w = wx[a] * wyz;
-            su += w * P.u[4 * b + a]; sv += w * P.v[4 * b + a]; sw += w * P.w[4 * b + a];
+        for (int c = 0; c < 3; c++) {
+            const float *v = comp[c];
+            float r[4];
+#pragma unroll
+            for (int b = 0; b < 4; b++)
+                r[b] = fmaf(wx[3], v[4 * b + 3], fmaf(wx[2], v[4 * b + 2], fmaf(wx[1], v[4 * b + 1], __fmul_rn(wx[0], v[4 * b]))));
+            const float t = __fmul_rn(wz[k], fmaf(wy[3], r[3], fmaf(wy[2], r[2], fmaf(wy[1], r[1], __fmul_rn(wy[0], r[0])))));
+            s[c] = k == 0 ? t : __fadd_rn(s[c], t);
         }
     }
 #pragma unroll
-    for (int o = 1; o <= 2; o <<= 1) {
-        su += __shfl_xor_sync(0xffffffffu, su, o);
-        sv += __shfl_xor_sync(0xffffffffu, sv, o);
-        sw += __shfl_xor_sync(0xffffffffu, sw, o);
-    }
-    ur = su; vr = sv; wr = sw;
+    for (int o = 1; o < LANES; o <<= 1)
+#pragma unroll
+        for (int c = 0; c < 3; c++) s[c] = __fadd_rn(s[c], __shfl_xor_sync(0xffffffffu, s[c], o));
 }
 
-constexpr int ADVECT_THREADS = 256;
 constexpr int ADVECT_MAX_PATCH = MAX_PATCH_VERTICES;
 constexpr int ADVECT_BOX_BYTES = 48 * 1024;
 constexpr int ADVECT_BOX_CAP = ADVECT_BOX_BYTES / (int)sizeof(float4);
@@ -445,12 +448,13 @@ __device__ __forceinline__ bool box_plane(const float4 *box, int bxs, int bys, i
 // stencil outside the box, gathers from global memory instead.
 // bid: the block's (cell, patch) index, blockIdx.x of a one-lattice launch.
 // RK: RUNGE_KUTTA, the stages of ibm.cu:430-517 (4), 518-574 (2) or 575-617 (1).
-template <bool XPER, int RK>
+template <bool XPER, int RK, int LANES>
 __device__ __forceinline__ void
 advect_body(const Geom &g, double *__restrict__ X, double *__restrict__ Xd, float *__restrict__ U,
             const float4 *__restrict__ uvr, long long nv, int V, const int *__restrict__ patch_off,
             const int *__restrict__ patch_vtx, int npatch, double dtM, int *__restrict__ flags, int bid)
 {
+    constexpr int ADVECT_THREADS = ADVECT_VERTICES * LANES, PLANES = 4 / LANES;
     extern __shared__ float4 abox[];   // [ADVECT_BOX_CAP] box, then the patch's positions and vertex ids
     double *spos = reinterpret_cast<double *>(abox + ADVECT_BOX_CAP);   // [3][ADVECT_MAX_PATCH]
     int *svid = reinterpret_cast<int *>(spos + 3 * ADVECT_MAX_PATCH);    // [ADVECT_MAX_PATCH]
@@ -528,102 +532,116 @@ advect_body(const Geom &g, double *__restrict__ X, double *__restrict__ Xd, floa
     }
     __syncthreads();
 
-    // four lanes per vertex (lane c owns stencil plane c), 64 vertices per pass;
-    // every lane of a warp runs the same passes (shuffles), idle lanes shadow vertex 0
-    const int c = tid & 3;
-    const int npass = (np + ADVECT_THREADS / 4 - 1) / (ADVECT_THREADS / 4);
+    // lane c of a vertex owns the stencil planes c PLANES ...; every lane of a
+    // warp runs the same passes (shuffles), idle lanes shadow vertex 0
+    const int c = tid % LANES;
+    const int npass = (np + ADVECT_VERTICES - 1) / ADVECT_VERTICES;
     for (int pass = 0; pass < npass; pass++) {
-        const int j = pass * (ADVECT_THREADS / 4) + (tid >> 2);
+        const int j = pass * ADVECT_VERTICES + tid / LANES;
         const bool live = j < np;
         const int jj = live ? j : 0;
-        const long long vj = vb + svid[jj];
-        const double xn = spos[jj], yn = spos[ADVECT_MAX_PATCH + jj], zn = spos[2 * ADVECT_MAX_PATCH + jj];
-        Plane16 P;
-        int bx, by, bz;
-        float fx, fy, fz, wx[4], wy[4], wz[4];
-        lattice_cell(g, xn, yn, zn, bx, by, bz, fx, fy, fz);
-        // shift from the raw z (and, periodic, x) frame to the cell's unwrapped frame
-        const double lzr = lat_z(g, zn);
-        const int zsh = (int)lrint(unwrap_near(lzr, az, g.nzc) - lzr);
-        const double lxr = lat_x(g, xn);
-        const int xsh = XPER ? (int)lrint(unwrap_near(lxr, ax, g.nx) - lxr) : 0;
+        Plane16 P[PLANES];
+        float wx[4], wy[4], wz4[4], wz[PLANES];
+        const double lxr = lat_x(g, spos[jj]), lyr = lat_y(g, spos[ADVECT_MAX_PATCH + jj]);
+        const double lzr = lat_z(g, spos[2 * ADVECT_MAX_PATCH + jj]);
+        const double flx = floor(lxr), fly = floor(lyr), flz = floor(lzr);
+        int bx = (int)flx - 1, by = (int)fly - 1, bz = (int)flz - 1;
+        float fx = (float)(lxr - flx), fy = (float)(lyr - fly), fz = (float)(lzr - flz);
+        // shift from the raw z (and, periodic, x) frame to the cell's unwrapped frame (unwrap_near)
+        auto frame_shift = [](double l, double ref, int n) { return l - ref > 0.5 * n ? -n : l - ref < -0.5 * n ? n : 0; };
+        const int zsh = frame_shift(lzr, az, g.nzc);
+        const int xsh = XPER ? frame_shift(lxr, ax, g.nx) : 0;
         auto fetch = [&](int cx, int cy, int cz) {
-            const int izr = cz + c;
-            const bool zin = izr >= -2 && izr < g.nzc + 2;   // beyond the BUFF planes (ibm.cu:453-455)
             unsigned xm = 0xFu;
-            if (XPER) {   // the same rule for the x BUFF columns (cx: raw frame)
+            if (XPER) {   // the same rule as for z (below) for the x BUFF columns (cx: raw frame)
                 xm = 0u;
 #pragma unroll
                 for (int a = 0; a < 4; a++) xm |= (cx + a >= -g.xb && cx + a < g.nx + g.xb) ? (1u << a) : 0u;
             }
-            if (!use_box || !box_plane(abox, bxs, bys, bzs, bps, cx + xsh - bx0, cy - by0, izr + zsh - bz0, zin, xm, P))
-                gather_plane(g, uvr, cx, cy, izr, xm, P);
+#pragma unroll
+            for (int k = 0; k < PLANES; k++) {
+                const int izr = cz + c * PLANES + k;
+                const bool zin = izr >= -2 && izr < g.nzc + 2;   // beyond the BUFF planes (ibm.cu:453-455)
+                if (!use_box || !box_plane(abox, bxs, bys, bzs, bps, cx + xsh - bx0, cy - by0, izr + zsh - bz0, zin, xm, P[k]))
+                    gather_plane(g, uvr, cx, cy, izr, xm, P[k]);
+            }
         };
         fetch(bx, by, bz);
         // the later stages' lattice positions relative to the stage-1 cell, in FP32:
         // x_k = x_n + u_{k-1} h moves the vertex by u h / dx lattice units (~1e-2)
         const int bx1 = bx, by1 = by, bz1 = bz;
         const float f1x = fx, f1y = fy, f1z = fz;
-        float us[RK], vs[RK], ws[RK];
+        float us[RK][3];
 #pragma unroll
         for (int k = 0; k < RK; k++) {
             if (k > 0) {
                 // RK4: x + u1 M dt / 2, x + u2 M dt / 2, x + u3 M dt (ibm.cu:487-505);
                 // RK2: x + u1 M (ibm.cu:560-562; dt = 1 there)
                 const float hs = (float)((RK == 4 && k < 3 ? 0.5 : 1.0) * dtM * g.inv_dx);
-                const float gxs = fmaf(us[k - 1], hs, f1x), gys = fmaf(vs[k - 1], hs, f1y), gzs = fmaf(ws[k - 1], hs, f1z);
+                const float gxs = fmaf(us[k - 1][0], hs, f1x), gys = fmaf(us[k - 1][1], hs, f1y), gzs = fmaf(us[k - 1][2], hs, f1z);
                 const float sx = floorf(gxs), sy = floorf(gys), sz = floorf(gzs);
                 fx = gxs - sx; fy = gys - sy; fz = gzs - sz;
                 const int cx = bx1 + (int)sx, cy = by1 + (int)sy, cz = bz1 + (int)sz;
-                if (cx != bx || cy != by || cz != bz) {   // uniform across the 4 lanes of the vertex
+                if (cx != bx || cy != by || cz != bz) {   // uniform across the lanes of the vertex
                     bx = cx; by = cy; bz = cz;
                     fetch(bx, by, bz);
                 }
             }
-            delta4(fx, wx); delta4(fy, wy); delta4(fz, wz);
-            const float wzc = c == 0 ? wz[0] : c == 1 ? wz[1] : c == 2 ? wz[2] : wz[3];
-            contract(P, wx, wy, wzc, us[k], vs[k], ws[k]);
+            delta4(fx, wx); delta4(fy, wy); delta4(fz, wz4);
+#pragma unroll
+            for (int i = 0; i < PLANES; i++) {
+                wz[i] = wz4[i];
+#pragma unroll
+                for (int l = 1; l < LANES; l++) if (c == l) wz[i] = wz4[l * PLANES + i];
+            }
+            contract<LANES>(P, wx, wy, wz, us[k]);
         }
-        if (!live || c != 0) continue;
-        double um, vm, wm;
-        if constexpr (RK == 4) {
-            um = ((double)us[0] + 2.0 * us[1] + 2.0 * us[2] + us[3]) / 6.0;
-            vm = ((double)vs[0] + 2.0 * vs[1] + 2.0 * vs[2] + vs[3]) / 6.0;
-            wm = ((double)ws[0] + 2.0 * ws[1] + 2.0 * ws[2] + ws[3]) / 6.0;
-        } else if constexpr (RK == 2) {   // ibm.cu:570-572
-            um = ((double)us[0] + (double)us[1]) / 2.0;
-            vm = ((double)vs[0] + (double)vs[1]) / 2.0;
-            wm = ((double)ws[0] + (double)ws[1]) / 2.0;
-        } else {                          // ibm.cu:614-616
-            um = us[0]; vm = vs[0]; wm = ws[0];
+        if (!live) continue;
+        // the move of the vertex, its components shared out over its lanes
+        const long long vj = vb + svid[jj];
+        bool finite = true;
+#pragma unroll
+        for (int m = 0; m < (3 + LANES - 1) / LANES; m++) {
+            const int d = m * LANES + c;
+            if (d >= 3) break;
+            float q[RK];
+#pragma unroll
+            for (int k = 0; k < RK; k++) q[k] = d == 0 ? us[k][0] : d == 1 ? us[k][1] : us[k][2];
+            double um;
+            if constexpr (RK == 4) um = ((double)q[0] + 2.0 * q[1] + 2.0 * q[2] + q[3]) / 6.0;
+            else if constexpr (RK == 2) um = ((double)q[0] + (double)q[1]) / 2.0;   // ibm.cu:570-572
+            else um = q[0];                                                          // ibm.cu:614-616
+            double r = __fma_rn(um, dtM, spos[d * ADVECT_MAX_PATCH + jj]);
+            if (d == 0) { if (r < g.xmin) r += g.LX; if (r > g.xmax) r -= g.LX; }   // ibm.cu:629-632
+            if (d == 2) { if (r < g.zmin) r += g.LZ; if (r > g.zmax) r -= g.LZ; }
+            finite = finite && isfinite(r);
+            X[d * nv + vj] = r;
+            Xd[d * nv + vj] = r;
+            U[d * nv + vj] = (float)um;
         }
-        double xr = xn + um * dtM, yr = yn + vm * dtM, zr = zn + wm * dtM;
-        if (xr < g.xmin) xr += g.LX;   // ibm.cu:629-632
-        if (xr > g.xmax) xr -= g.LX;
-        if (zr < g.zmin) zr += g.LZ;
-        if (zr > g.zmax) zr -= g.LZ;
-        if (!isfinite(xr) || !isfinite(yr) || !isfinite(zr)) atomicOr(flags, RBC_FLAG_NONFINITE);
-        X[vj] = xr; X[nv + vj] = yr; X[2 * nv + vj] = zr;
-        Xd[vj] = xr; Xd[nv + vj] = yr; Xd[2 * nv + vj] = zr;
-        U[vj] = (float)um; U[nv + vj] = (float)vm; U[2 * nv + vj] = (float)wm;
+        if (!finite) atomicOr(flags, RBC_FLAG_NONFINITE);
     }
 }
 
-template <bool XPER, int RK>
-__global__ void __launch_bounds__(ADVECT_THREADS)
+// resident blocks per multiprocessor the register allocation must allow
+constexpr int advect_min_blocks(int lanes) { return lanes == 2 ? 3 : 2; }
+
+template <bool XPER, int RK, int LANES>
+__global__ void __launch_bounds__(ADVECT_VERTICES * LANES, advect_min_blocks(LANES))
 advect_kernel(const Geom g, double *__restrict__ X, double *__restrict__ Xd, float *__restrict__ U,
               const float4 *__restrict__ uvr, long long nv, int V, const int *__restrict__ patch_off,
               const int *__restrict__ patch_vtx, int npatch, double dtM, int *__restrict__ flags)
 {
     pdl_start();
-    advect_body<XPER, RK>(g, X, Xd, U, uvr, nv, V, patch_off, patch_vtx, npatch, dtM, flags, blockIdx.x);
+    advect_body<XPER, RK, LANES>(g, X, Xd, U, uvr, nv, V, patch_off, patch_vtx, npatch, dtM, flags, blockIdx.x);
 }
 
 cudaError_t advect_setup()
 {
-    const void *ks[] = {(const void *)advect_kernel<false, 4>, (const void *)advect_kernel<true, 4>,
-                        (const void *)advect_kernel<false, 2>, (const void *)advect_kernel<true, 2>,
-                        (const void *)advect_kernel<false, 1>, (const void *)advect_kernel<true, 1>};
+    const void *ks[] = {(const void *)advect_kernel<false, 4, 4>, (const void *)advect_kernel<true, 4, 4>,
+                        (const void *)advect_kernel<false, 4, 2>, (const void *)advect_kernel<true, 4, 2>,
+                        (const void *)advect_kernel<false, 2, 4>, (const void *)advect_kernel<true, 2, 4>,
+                        (const void *)advect_kernel<false, 1, 4>, (const void *)advect_kernel<true, 1, 4>};
     for (const void *k : ks) {
         const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, ADVECT_SMEM);
         if (e != cudaSuccess) return e;
@@ -631,13 +649,19 @@ cudaError_t advect_setup()
     return cudaSuccess;
 }
 
+// more blocks than are resident at once with four lanes (two per multiprocessor)
+static bool advect_two_lanes(long long blocks, int sms) { return blocks > 2LL * sms; }
+
 void launch_advect(const Geom &g, const AdvectArgs &a, cudaStream_t s)
 {
     if (a.ncell <= 0) return;
-    auto k = a.rk == 1 ? (g.xper ? advect_kernel<true, 1> : advect_kernel<false, 1>)
-           : a.rk == 2 ? (g.xper ? advect_kernel<true, 2> : advect_kernel<false, 2>)
-                       : (g.xper ? advect_kernel<true, 4> : advect_kernel<false, 4>);
-    launch_pdl(k, dim3(a.ncell * a.npatch), dim3(ADVECT_THREADS), ADVECT_SMEM, s,
+    // the lower orders, with a stage or two, keep four lanes
+    const bool two = a.rk == 4 && advect_two_lanes((long long)a.ncell * a.npatch, a.sms);
+    auto k = a.rk == 1 ? (g.xper ? advect_kernel<true, 1, 4> : advect_kernel<false, 1, 4>)
+           : a.rk == 2 ? (g.xper ? advect_kernel<true, 2, 4> : advect_kernel<false, 2, 4>)
+           : two       ? (g.xper ? advect_kernel<true, 4, 2> : advect_kernel<false, 4, 2>)
+                       : (g.xper ? advect_kernel<true, 4, 4> : advect_kernel<false, 4, 4>);
+    launch_pdl(k, dim3(a.ncell * a.npatch), dim3(ADVECT_VERTICES * (two ? 2 : 4)), ADVECT_SMEM, s,
                g, a.X, a.Xd, a.U, a.uvr, a.nv, a.V, a.patch_off, a.patch_vtx, a.npatch, a.dtM, a.flags);
 }
 
@@ -654,14 +678,14 @@ spread_fused_kernel(const DomainArgs *__restrict__ dom, const int *__restrict__ 
                       a.flags, blockIdx.x - boff[d]);
 }
 
-template <bool XPER>
-__global__ void __launch_bounds__(ADVECT_THREADS)
+template <bool XPER, int LANES>
+__global__ void __launch_bounds__(ADVECT_VERTICES * LANES, advect_min_blocks(LANES))
 advect_fused_kernel(const DomainArgs *__restrict__ dom, const int *__restrict__ boff, int ndom)
 {
     const int d = fused_domain(boff, ndom, blockIdx.x);
     const DomainArgs &D = dom[d];
     const AdvectArgs &a = D.adv;
-    advect_body<XPER, 4>(D.g, a.X, a.Xd, a.U, a.uvr, a.nv, a.V, a.patch_off, a.patch_vtx, a.npatch, a.dtM, a.flags,
+    advect_body<XPER, 4, LANES>(D.g, a.X, a.Xd, a.U, a.uvr, a.nv, a.V, a.patch_off, a.patch_vtx, a.npatch, a.dtM, a.flags,
                       blockIdx.x - boff[d]);
 }
 
@@ -672,7 +696,8 @@ cudaError_t ibm_fused_setup()
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SPREAD_SMEM);
         if (e != cudaSuccess) return e;
     }
-    const void *ka[] = {(const void *)advect_fused_kernel<false>, (const void *)advect_fused_kernel<true>};
+    const void *ka[] = {(const void *)advect_fused_kernel<false, 4>, (const void *)advect_fused_kernel<true, 4>,
+                        (const void *)advect_fused_kernel<false, 2>, (const void *)advect_fused_kernel<true, 2>};
     for (const void *k : ka) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, ADVECT_SMEM);
         if (e != cudaSuccess) return e;
@@ -687,11 +712,13 @@ void launch_spread_fused(const FusedLaunch &f, bool xper, cudaStream_t s)
     k<<<f.nblocks, SPREAD_THREADS, SPREAD_SMEM, s>>>(f.dom, f.boff, f.ndom);
 }
 
-void launch_advect_fused(const FusedLaunch &f, bool xper, cudaStream_t s)
+void launch_advect_fused(const FusedLaunch &f, bool xper, int sms, cudaStream_t s)
 {
     if (f.nblocks <= 0) return;
-    auto k = xper ? advect_fused_kernel<true> : advect_fused_kernel<false>;
-    k<<<f.nblocks, ADVECT_THREADS, ADVECT_SMEM, s>>>(f.dom, f.boff, f.ndom);
+    const bool two = advect_two_lanes(f.nblocks, sms);
+    auto k = two ? (xper ? advect_fused_kernel<true, 2> : advect_fused_kernel<false, 2>)
+                 : (xper ? advect_fused_kernel<true, 4> : advect_fused_kernel<false, 4>);
+    k<<<f.nblocks, ADVECT_VERTICES * (two ? 2 : 4), ADVECT_SMEM, s>>>(f.dom, f.boff, f.ndom);
 }
 
 }  // namespace rbc

@@ -883,7 +883,7 @@ AdvectArgs advect_args(rbc_handle *h, CellGroup &g)
     AdvectArgs a{};
     a.X = g.X; a.Xd = g.Xd; a.U = g.U; a.uvr = h->uvr; a.nv = g.nv;
     a.V = g.V; a.ncell = g.ncell; a.patch_off = g.patch_off; a.patch_vtx = g.patch_vtx; a.npatch = g.npatch;
-    a.dtM = h->p.dt * h->p.M; a.rk = h->p.rk_order; a.flags = h->d_flags();
+    a.dtM = h->p.dt * h->p.M; a.rk = h->p.rk_order; a.sms = h->sms; a.flags = h->d_flags();
     return a;
 }
 
@@ -1277,7 +1277,7 @@ int batch_build_fused(rbc_batch *b)
         launch_spread_fused(f[FS_SPREAD], xper, b->stream);
         launch_lbm_fused(f[FS_LBM], h0->p.storage, off32, tpb, b->stream);
         launch_clear_bits_fused(f[FS_CLEAR], b->stream);   // the force reset after the read
-        launch_advect_fused(f[FS_ADVECT], xper, b->stream);
+        launch_advect_fused(f[FS_ADVECT], xper, h0->sms, b->stream);
         launch_volume_fused(f[FS_VOLUME], V, b->stream);
         const cudaError_t le = cudaGetLastError();
         const cudaError_t e = cudaStreamEndCapture(b->stream, &graph);

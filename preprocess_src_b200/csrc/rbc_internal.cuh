@@ -271,6 +271,7 @@ struct AdvectArgs {
     int npatch;
     double dtM;                // dt * M
     int rk;                    // RUNGE_KUTTA: 1, 2 or 4 stages
+    int sms;                   // multiprocessors of the device
     int *flags;
 };
 void launch_advect(const Geom &g, const AdvectArgs &a, cudaStream_t s);
@@ -516,7 +517,7 @@ void launch_clear_bits_fused(const FusedLaunch &f, cudaStream_t s);   // the for
 void launch_membrane_fused(const FusedLaunch &f, bool fp64, int V, int vpt, cudaStream_t s);   // a block per cell
 void launch_spread_fused(const FusedLaunch &f, bool xper, cudaStream_t s);    // a block per (cell, patch)
 void launch_lbm_fused(const FusedLaunch &f, int storage, bool off32, int threads, cudaStream_t s);
-void launch_advect_fused(const FusedLaunch &f, bool xper, cudaStream_t s);    // a block per (cell, patch)
+void launch_advect_fused(const FusedLaunch &f, bool xper, int sms, cudaStream_t s);    // a block per (cell, patch)
 void launch_volume_fused(const FusedLaunch &f, int V, cudaStream_t s);        // a block per cell
 int  membrane_threads(int V, int vpt);     // threads of a membrane block with vpt vertices per thread
 int  membrane_default_vpt(int V);          // the vertices per thread of a one-population launch
