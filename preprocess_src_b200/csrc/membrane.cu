@@ -1,4 +1,4 @@
-// membrane.cu -- Skalak membrane FEM nodal forces, one CTA per cell.
+// membrane.cu -- Skalak membrane FEM nodal forces, one CTA (or cluster of CTAs) per cell.
 //
 // Replaces calc_tension, calc_load (with its per-cell BiCGSTAB) and q2f
 // (stress.cu:29-445, matrix_solver.cu:279-377 of the reference).  The
@@ -53,6 +53,10 @@
 // (Real); the solve runs in FP32.
 #include "rbc_internal.cuh"
 
+#include <cooperative_groups.h>
+
+namespace cg = cooperative_groups;
+
 namespace rbc {
 
 constexpr int MEM_MAX_THREADS = 1024;
@@ -93,10 +97,11 @@ __device__ __forceinline__ void store_vec4(double4 *p, const double4 &v) {
     double2 *q = reinterpret_cast<double2 *>(p);
     q[0] = make_double2(v.x, v.y); q[1] = make_double2(v.z, v.w);
 }
-__device__ __forceinline__ float4 load_vec4(const float4 *p) { return *p; }
-__device__ __forceinline__ double4 load_vec4(const double4 *p) {
+// OWN: written by this block; else by another block of the cluster, read past the L1
+template <bool OWN> __device__ __forceinline__ float4 load_vec4(const float4 *p) { return OWN ? *p : __ldcg(p); }
+template <bool OWN> __device__ __forceinline__ double4 load_vec4(const double4 *p) {
     const double2 *q = reinterpret_cast<const double2 *>(p);
-    const double2 x = q[0], y = q[1];
+    const double2 x = OWN ? q[0] : __ldcg(q), y = OWN ? q[1] : __ldcg(q + 1);
     return make_double4(x.x, x.y, y.x, y.y);
 }
 
@@ -106,13 +111,24 @@ constexpr int MAX_VALENCE = 6;   // checked when the topology is built
 // registers a thread), 1024 otherwise
 template <int VPT> constexpr int mem_max_threads() { return VPT >= 3 ? 896 : MEM_MAX_THREADS; }
 
-// cell: the block's cell, blockIdx.x of a one-population launch
-template <typename Real, int VPT>
+// A cell is one block's work (CL = 1) or a cluster's of CL blocks.  In a cluster
+// block `rank` owns a CL-th of the elements and of the solve positions (contiguous:
+// rings of the breadth-first order).  Records cross through the L2-resident scratch;
+// in the solve every block keeps the whole d vector in its own shared memory and
+// stores each new value also into the blocks that own a neighbour of the vertex
+// (those are the ones that read it), one cluster barrier per iteration.  A vertex's
+// arithmetic does not depend on CL, so the forces are the same bit for bit.
+// cell: the block's cell, blockIdx.x / CL of a one-population launch
+template <typename Real, int VPT, int CL = 1>
 __device__ __forceinline__ void membrane_body(const MembraneArgs &a, int cell)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ float red[32];
     const int V = a.V, E = a.E, tid = threadIdx.x, T = blockDim.x;
+    const int rank = CL > 1 ? (int)cg::this_cluster().block_rank() : 0;
+    auto barrier = [] { if constexpr (CL > 1) { __syncwarp(); cg::this_cluster().sync(); } else __syncthreads(); };
+    const int share = (V + CL - 1) / CL, P0 = rank * share, P1 = min(V, P0 + share);   // the block's solve positions
+    const int eshare = (E + CL - 1) / CL, E0 = rank * eshare, E1 = min(E, E0 + eshare);
     double *pos = reinterpret_cast<double *>(smem);                    // [3][V]
     float *dbuf = reinterpret_cast<float *>(smem);                     // [2][3][V], after assembly
     float *coef = reinterpret_cast<float *>(smem + 32 * (size_t)V);    // [6][V]
@@ -130,7 +146,7 @@ __device__ __forceinline__ void membrane_body(const MembraneArgs &a, int cell)
     const Real C = (Real)a.C, rgs = (Real)a.rgs;
     using R4 = typename Vec4<Real>::T;
     R4 *rec = reinterpret_cast<R4 *>(a.erec) + (size_t)eb * 3;   // [E][3 slots]: load on the slot's vertex, gab
-    for (int e = tid; e < E; e += T) {
+    for (int e = E0 + tid; e < E1; e += T) {
         const int ia = __ldg(&a.tri[3 * e]), ib = __ldg(&a.tri[3 * e + 1]), ic = __ldg(&a.tri[3 * e + 2]);
         const double e1x = mimage(pos[ib] - pos[ia], a.LX), e1y = pos[V + ib] - pos[V + ia];
         const double e1z = mimage(pos[2 * V + ib] - pos[2 * V + ia], a.LZ);
@@ -183,18 +199,18 @@ __device__ __forceinline__ void membrane_body(const MembraneArgs &a, int cell)
         store_vec4(rec + (size_t)3 * e + 1, make_vec4(bx, by, bz, gab));
         store_vec4(rec + (size_t)3 * e + 2, make_vec4(cx, cy, cz, gab));
     }
-    __syncthreads();   // the records are written by this CTA and read below (plain loads, not __ldg)
+    barrier();   // the records are written by this block (its cluster) and read below (no __ldg)
 
     // vertex pass: matrix row, right-hand side and nodal area of each vertex.
-    // Thread tid owns solve positions p = tid + m T, the vertex vord[p] at each.
+    // Thread tid owns solve positions p = P0 + tid + m T, the vertex vord[p] at each.
     float rhs[VPT][3], ds[VPT];
     int vid[VPT];
 #pragma unroll
     for (int m = 0; m < VPT; m++) {
-        const int p = tid + m * T;
+        const int p = P0 + tid + m * T;
         rhs[m][0] = rhs[m][1] = rhs[m][2] = 0.f; ds[m] = 0.f;
         vid[m] = 0;
-        if (p >= V) continue;
+        if (p >= P1) continue;
         const int i = __ldg(&a.vord[p]);
         vid[m] = i;
         Real diag = 0, off[6] = {0, 0, 0, 0, 0, 0}, b0 = 0, b1 = 0, b2 = 0, dsum = 0;
@@ -206,7 +222,7 @@ __device__ __forceinline__ void membrane_body(const MembraneArgs &a, int cell)
         R4 r[MAX_VALENCE];
 #pragma unroll
         for (int j = 0; j < MAX_VALENCE; j++)
-            if (k0 + j < k1) r[j] = load_vec4(rec + (size_t)3 * v2e_elem(pk[j]) + v2e_en(pk[j]));
+            if (k0 + j < k1) r[j] = load_vec4<CL == 1>(rec + (size_t)3 * v2e_elem(pk[j]) + v2e_en(pk[j]));
 #pragma unroll
         for (int j = 0; j < MAX_VALENCE; j++) {
             if (k0 + j >= k1) break;
@@ -232,31 +248,49 @@ __device__ __forceinline__ void membrane_body(const MembraneArgs &a, int cell)
     float rho = 1.0f / sigma, bb = 0.f;
 #pragma unroll
     for (int m = 0; m < VPT; m++) {
-        const int p = tid + m * T;
+        const int p = P0 + tid + m * T;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             x[m][c] = 0.f; r[m][c] = rhs[m][c]; d[m][c] = rhs[m][c] / theta;
             bb += rhs[m][c] * rhs[m][c];
         }
-        if (p < V) { dbuf[p] = d[m][0]; dbuf[V + p] = d[m][1]; dbuf[2 * V + p] = d[m][2]; }
+        if (p < P1) { dbuf[p] = d[m][0]; dbuf[V + p] = d[m][1]; dbuf[2 * V + p] = d[m][2]; }
     }
     // each vertex's neighbours and row coefficients stay in registers for the
     // whole solve (a missing sixth neighbour points at the vertex itself with
     // coefficient 0)
     unsigned nb[VPT][3];   // two 16-bit neighbour ids per register
     float cf[VPT][6];
+    unsigned rem[VPT];     // CL > 1: the other blocks that read the vertex's value
 #pragma unroll
     for (int m = 0; m < VPT; m++) {
-        const int p = tid + m * T;
+        const int p = P0 + tid + m * T;
+        rem[m] = 0u;
 #pragma unroll
         for (int s = 0; s < 6; s++) {
-            const int j = p < V ? (int)__ldg(&a.nbrp[s * V + p]) : -1;   // neighbours by solve position
-            const unsigned id = (unsigned)(j >= 0 ? j : (p < V ? p : 0));
+            const int j = p < P1 ? (int)__ldg(&a.nbrp[s * V + p]) : -1;   // neighbours by solve position
+            const unsigned id = (unsigned)(j >= 0 ? j : (p < P1 ? p : 0));
             if (s & 1) nb[m][s >> 1] |= id << 16; else nb[m][s >> 1] = id;
             cf[m][s] = j >= 0 ? coef[s * V + p] : 0.f;
+            if (CL > 1 && j >= 0) rem[m] |= 1u << (j / share);
         }
+        if (CL > 1) rem[m] &= ~(1u << rank);
     }
-    __syncthreads();
+    // the value at position p (m of this thread) into the same buffer of the blocks that read it
+    auto send = [&](float *to, int m, int p) {
+#pragma unroll
+        for (int o = 0; o < CL; o++)
+            if ((rem[m] >> o) & 1u) {
+                float *far = cg::this_cluster().map_shared_rank(to, o);
+                far[p] = d[m][0]; far[V + p] = d[m][1]; far[2 * V + p] = d[m][2];
+            }
+    };
+    if constexpr (CL > 1) {
+#pragma unroll
+        for (int m = 0; m < VPT; m++)
+            if (P0 + tid + m * T < P1) send(dbuf, m, P0 + tid + m * T);
+    }
+    barrier();
     for (int it = 0; it < a.niter; it++) {
         // one array per component: three 4-byte gathers per neighbour, whose
         // warp-wide reads of nearby positions take one wavefront each
@@ -266,8 +300,8 @@ __device__ __forceinline__ void membrane_body(const MembraneArgs &a, int cell)
         const float c1 = rho_n * rho, c2 = 2.0f * rho_n / delta;
 #pragma unroll
         for (int m = 0; m < VPT; m++) {
-            const int p = tid + m * T;
-            if (p >= V) continue;
+            const int p = P0 + tid + m * T;
+            if (p >= P1) continue;
             float ad0 = d[m][0], ad1 = d[m][1], ad2 = d[m][2];
 #pragma unroll
             for (int s = 0; s < 6; s++) {
@@ -280,25 +314,37 @@ __device__ __forceinline__ void membrane_body(const MembraneArgs &a, int cell)
 #pragma unroll
             for (int c = 0; c < 3; c++) d[m][c] = c1 * d[m][c] + c2 * r[m][c];
             nxt[p] = d[m][0]; nxt[V + p] = d[m][1]; nxt[2 * V + p] = d[m][2];
+            if constexpr (CL > 1) send(nxt, m, p);
         }
         rho = rho_n;
-        __syncthreads();
+        barrier();   // the last one also keeps every block until no other stores into it
     }
     // residual of the scaled system, relative to its right-hand side: the flag
     // is |r| / |b| > 1e-3, compared as squared norms
     float rr = 0.f;
 #pragma unroll
     for (int m = 0; m < VPT; m++)
-        if (tid + m * T < V)
+        if (P0 + tid + m * T < P1)
 #pragma unroll
             for (int c = 0; c < 3; c++) rr += r[m][c] * r[m][c];
     rr = block_sum(rr, red);
     bb = block_sum(bb, red);
-    if (tid == 0 && rr > 1e-6f * bb && a.flags) atomicOr(a.flags, RBC_FLAG_SOLVE_RESIDUAL);
+    if constexpr (CL > 1) {   // the cell's sums in its first block
+        __shared__ float part[2][CL];
+        if (tid == 0) {
+            cg::this_cluster().map_shared_rank(&part[0][0], 0)[rank] = rr;
+            cg::this_cluster().map_shared_rank(&part[0][0], 0)[CL + rank] = bb;
+        }
+        barrier();
+        rr = bb = 0.f;
+        if (rank == 0)
+            for (int o = 0; o < CL; o++) { rr += part[0][o]; bb += part[1][o]; }
+    }
+    if (tid == 0 && rank == 0 && rr > 1e-6f * bb && a.flags) atomicOr(a.flags, RBC_FLAG_SOLVE_RESIDUAL);
     // q2f (stress.cu:440-442)
 #pragma unroll
     for (int m = 0; m < VPT; m++) {
-        if (tid + m * T >= V) continue;
+        if (P0 + tid + m * T >= P1) continue;
         const int i = vid[m];
         a.Fv[vb + i] = -x[m][0] * ds[m];
         a.Fv[nv + vb + i] = -x[m][1] * ds[m];
@@ -314,27 +360,39 @@ membrane_kernel(const MembraneArgs a)
     membrane_body<Real, VPT>(a, blockIdx.x);
 }
 
-template <typename Real, int VPT>
+template <typename Real, int VPT, int CL>
+__global__ void __launch_bounds__(mem_max_threads<VPT>(), 1)
+membrane_cluster_kernel(const MembraneArgs a)
+{
+    pdl_start();
+    membrane_body<Real, VPT, CL>(a, blockIdx.x / CL);
+}
+
+template <typename Real, int VPT, int CL = 1>
 static void launch_vpt(const MembraneArgs &a, cudaStream_t s)
 {
     const int smem = membrane_smem_bytes(a.V);
-    auto k = membrane_kernel<Real, VPT>;
-    int T = (a.V + VPT - 1) / VPT;
+    void (*k)(MembraneArgs);
+    if constexpr (CL > 1) k = membrane_cluster_kernel<Real, VPT, CL>; else k = membrane_kernel<Real, VPT>;
+    int T = ((a.V + CL - 1) / CL + VPT - 1) / VPT;
     T = ((T + 31) / 32) * 32;
     // launched at the given stream priority: when the previous step's volume
     // correction runs beside it, the membrane CTAs are dispatched first
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)a.ncell);
+    cfg.gridDim = dim3((unsigned)(CL * a.ncell));
     cfg.blockDim = dim3((unsigned)T);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[3];
     attr[0].id = cudaLaunchAttributePriority;
     attr[0].val.priority = a.priority;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
+    attr[2].id = cudaLaunchAttributeClusterDimension;
+    attr[2].val.clusterDim.x = CL;
+    attr[2].val.clusterDim.y = attr[2].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = CL > 1 ? 3 : 2;
     cudaLaunchKernelEx(&cfg, k, a);
 }
 
@@ -343,6 +401,12 @@ static void launch_real(const MembraneArgs &a, cudaStream_t s)
 {
     // fewest vertices per thread whose CTA (rounded to warps) fits the thread cap
     auto fits = [&](int vpt, int cap) { return ((a.V + vpt - 1) / vpt + 31) / 32 * 32 <= cap; };
+    // few cells of many vertices leave most multiprocessors idle: a cluster per cell.  Up to 1024
+    // vertices one block's solve iteration is as short as a cluster barrier.  One kernel of cells of
+    // 2562 vertices: 64 us with one block each, 48 with two, 34 with four; the lines are where all
+    // clusters run at once (one block per multiprocessor, a cluster inside one group of them).
+    if (a.V > MEM_MAX_THREADS && 5 * a.ncell <= a.sms) { launch_vpt<Real, 1, 4>(a, s); return; }
+    if (a.V > MEM_MAX_THREADS && 2 * a.ncell <= a.sms) { launch_vpt<Real, 2, 2>(a, s); return; }
     if (fits(1, mem_max_threads<1>())) launch_vpt<Real, 1>(a, s);
     else if (fits(2, mem_max_threads<2>())) launch_vpt<Real, 2>(a, s);
     else if (fits(3, mem_max_threads<3>())) launch_vpt<Real, 3>(a, s);
@@ -357,7 +421,9 @@ cudaError_t membrane_setup(int optin, int *max_bytes)
     const void *ks[] = {(const void *)membrane_kernel<float, 1>, (const void *)membrane_kernel<float, 2>,
                         (const void *)membrane_kernel<float, 3>, (const void *)membrane_kernel<float, 4>,
                         (const void *)membrane_kernel<double, 1>, (const void *)membrane_kernel<double, 2>,
-                        (const void *)membrane_kernel<double, 3>, (const void *)membrane_kernel<double, 4>};
+                        (const void *)membrane_kernel<double, 3>, (const void *)membrane_kernel<double, 4>,
+                        (const void *)membrane_cluster_kernel<float, 1, 4>, (const void *)membrane_cluster_kernel<double, 1, 4>,
+                        (const void *)membrane_cluster_kernel<float, 2, 2>, (const void *)membrane_cluster_kernel<double, 2, 2>};
     int lo = optin;
     for (const void *k : ks) {
         int g = 0;

@@ -714,6 +714,8 @@ int launch_membrane_range(rbc_handle *h, CellGroup &g, int c0, int c1, cudaStrea
     a.niter = h->p.solver_iters > 0 ? h->p.solver_iters : DEFAULT_SOLVER_ITERS;
     a.flags = h->d_flags();
     a.priority = h->prio_high;
+    a.sms = 0;   // one block per cell: clusters would end this wave sooner, on multiprocessors the spread uses
+                 // beside it (dense suspension 427 -> 434 us a step)
     launch_membrane(a, h->p.membrane_fp64 != 0, st);
     h->launches++;
     CK_LAUNCH();
@@ -757,6 +759,7 @@ MembraneArgs membrane_args(rbc_handle *h, CellGroup &g)
     a.niter = h->p.solver_iters > 0 ? h->p.solver_iters : DEFAULT_SOLVER_ITERS;
     a.flags = h->d_flags();
     a.priority = h->prio_high;
+    a.sms = h->sms;
     return a;
 }
 

@@ -290,6 +290,7 @@ struct MembraneArgs {
     int niter;
     int *flags;
     int priority;             // launch priority (cudaLaunchAttributePriority)
+    int sms;                  // multiprocessors of the device; 0 = one block per cell whatever their number
 };
 int  membrane_smem_bytes(int V);
 int  membrane_limit_bytes(int V);   // bytes per block that bound the vertices per cell
