@@ -451,18 +451,22 @@ void launch_force_reset(const Geom &g, const ForceField &F, cudaStream_t s)
 // along opp p) and f3 = f*_p(i).  The weights sum to 1, so the same holds for
 // g = f - w.  No listed link reads a slot another one writes (a slot is
 // written only by its own node's link, and links with walls on both sides
-// are not listed).  One thread per (link, plane).
+// are not listed).  One thread per (link, plane); started early like the step's other
+// kernels, its link tables read before it waits (a tube of 220 x 77 x 77, 60 steps:
+// 4218 -> 4166 us).
 template <int STORE>
 __global__ void tube_bounce_kernel(const Geom g, typename Store<STORE>::T *__restrict__ gs,
                                    const int *__restrict__ links, const float *__restrict__ frac, int nlinks,
                                    float inv_scale, float scale)
 {
     using S = Store<STORE>;
+    pdl_launch();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nlinks) return;
     const int z = blockIdx.y;
     const int code = __ldg(&links[k]), xy = code >> 5, p = code & 31, o = opp(p);
     const float t = __ldg(&frac[k]);
+    pdl_wait();   // the links are the handle's own tables; the populations are the collide-stream's
     const long long zb = (long long)z * g.plane, i = zb + xy;
     const int zn = wrap_z(z + ez(p), g.nzc), dxy = ex(p) + g.nx * ey(p);   // node i + e_p
     typename S::T *slot = gs + (long long)o * g.nint + i;
@@ -484,9 +488,9 @@ void launch_tube_bounce(const Geom &g, int storage, void *gout, const int *links
     if (nlinks <= 0) return;
     const dim3 grid((unsigned)((nlinks + 127) / 128), (unsigned)g.nzc);
     if (storage == RBC_STORE_F16)
-        tube_bounce_kernel<RBC_STORE_F16><<<grid, 128, 0, s>>>(g, (__half *)gout, links, frac, nlinks, inv_scale, scale);
+        launch_pdl(tube_bounce_kernel<RBC_STORE_F16>, grid, dim3(128), 0, s, g, (__half *)gout, links, frac, nlinks, inv_scale, scale);
     else
-        tube_bounce_kernel<RBC_STORE_F32><<<grid, 128, 0, s>>>(g, (float *)gout, links, frac, nlinks, inv_scale, scale);
+        launch_pdl(tube_bounce_kernel<RBC_STORE_F32>, grid, dim3(128), 0, s, g, (float *)gout, links, frac, nlinks, inv_scale, scale);
 }
 
 // ---- reference layout <-> internal layout ---------------------------------

@@ -36,11 +36,10 @@ namespace rbc {
 // kernel first lets its own successor do the same, then waits until the
 // predecessor has completed and its writes are visible, before it touches
 // memory.  Without the launch attribute both instructions return at once.
-__device__ __forceinline__ void pdl_start()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// What no kernel writes (a handle's tables) may be read between the two.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_start() { pdl_launch(); pdl_wait(); }
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                               Args &&...args)
