@@ -2753,6 +2753,10 @@ int adjoint_reserve(rbc_handle *h, int K, int nseg)
     TRYA(adj_alloc(h, &a->pbar, 4)); TRYA(adj_alloc(h, &a->status, 1));
     TRYA(adj_alloc(h, &a->fin_uvr, n)); TRYA(adj_alloc(h, &a->fin_U, nv3)); TRYA(adj_alloc(h, &a->fin_Fv, nv3));
 #undef TRYA
+    // the velocity slots' wall nodes as the handle's field has them: the collide-stream stores
+    // nothing for a warp of wall nodes alone, and the interpolations at a wall read those nodes
+    launch_fill_f4(a->suvr, (long long)(S * n), make_float4(0.f, 0.f, 0.f, 1.f), h->stream);
+    CK_LAUNCH();
     a->K_cap = K;
     a->nseg_cap = nseg;
     return RBC_OK;
