@@ -3268,6 +3268,8 @@ int rbc_adjoint_backward(rbc_handle *h, const double *xbar, const double *ybar, 
 int rbc_set_coefficients(rbc_handle *h, double P, double B, double C)
 {
     if (!h || !std::isfinite(P) || !std::isfinite(B) || !std::isfinite(C)) return RBC_ERR_ARG;
+    // volume and area are the last recomputed segment's (a binomial sweep's own steps mark them valid)
+    h->metrics_valid = false;
     RBC_DEVICE_GUARD(h);
     CK(cudaStreamSynchronize(h->stream));
     h->p.P = P; h->p.B = B; h->p.C = C;
