@@ -1737,7 +1737,9 @@ int rbc_import_ref_lattice(rbc_handle *h, const double *fn)
 
 // The device's address of n doubles of the caller's page-locked memory, which a
 // kernel can write directly over the host link; NULL unless all of them lie in one
-// page-locked range that this device maps (and are aligned as a kernel needs them).
+// page-locked range that this device maps for reading and writing (memory can be
+// registered read-only, and a kernel's store to it would fault) and are aligned as
+// a kernel needs them.
 static double *mapped(double *p, size_t n)
 {
     using Query = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
@@ -1752,13 +1754,17 @@ static double *mapped(double *p, size_t n)
         return (Query)f;
     }();
     if (!query || !p || n == 0 || (uintptr_t)p % sizeof(double)) return nullptr;
-    CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
-                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                   CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
     unsigned type = 0;
     CUdeviceptr dev = 0, start = 0;
     size_t size = 0;
-    void *out[4] = {&type, &dev, &start, &size};
-    if (query(4, what, out, (CUdeviceptr)p) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || !dev) return nullptr;
+    unsigned long long access = 0;
+    void *out[5] = {&type, &dev, &start, &size, &access};
+    if (query(5, what, out, (CUdeviceptr)p) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || !dev ||
+        access != CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE)
+        return nullptr;
     const CUdeviceptr at = (CUdeviceptr)p;
     return start <= at && at + n * sizeof(double) <= start + size ? (double *)dev : nullptr;
 }
