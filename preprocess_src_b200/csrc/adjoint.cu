@@ -257,45 +257,41 @@ __device__ __forceinline__ bool sane_pos(const Geom &g, double px, double py, do
 
 constexpr int VTX_ADJ_THREADS = 128;   // four vertices per CTA, one warp each
 
-// One RK stage's stencil with the velocity at the lane's two nodes, kept from the
-// replay of the stages for their reversal: the FP64 sines and cosines, the weights
-// and the loads are the cost of a stage, and each is needed twice (642 vertices:
-// 14.4 -> 12.3 us).
-struct StageStencil {
-    LaneStencil s;
-    float3 q[2];
-};
-
 // Velocity of the frozen field at p as the forward advection interpolates it
 // (every lane returns the same sum).
 __device__ __forceinline__ void warp_interp(const Geom &g, const float4 *__restrict__ uvr, const double p[3], int lane,
-                                            StageStencil &st, double u[3]) {
-    lane_stencil(g, p[0], p[1], p[2], lane, st.s);
+                                            double u[3]) {
+    LaneStencil s;
+    lane_stencil(g, p[0], p[1], p[2], lane, s);
     double u0 = 0.0, u1 = 0.0, u2 = 0.0;
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const float4 q = st.s.n[h] >= 0 ? __ldg(&uvr[st.s.n[h]]) : make_float4(0.f, 0.f, 0.f, 0.f);
-        st.q[h] = make_float3(q.x, q.y, q.z);
-        u0 += st.s.w[h] * q.x; u1 += st.s.w[h] * q.y; u2 += st.s.w[h] * q.z;
-    }
+    for (int h = 0; h < 2; h++)
+        if (s.n[h] >= 0) {
+            const float4 q = __ldg(&uvr[s.n[h]]);
+            u0 += s.w[h] * q.x; u1 += s.w[h] * q.y; u2 += s.w[h] * q.z;
+        }
     u[0] = warp_sum(u0); u[1] = warp_sum(u1); u[2] = warp_sum(u2);
 }
 
-// Adjoint of one interpolation with output adjoint kb: adds w_n kb to the
-// velocity adjoint of each stencil node; returns in pb (every lane) the
+// Adjoint of one interpolation at p with output adjoint kb: adds w_n kb to
+// the velocity adjoint of each stencil node; returns in pb (every lane) the
 // position adjoint sum_n (d w_n / d p) (u_n . kb).
-__device__ __forceinline__ void warp_interp_adjoint(float *__restrict__ ubar, const StageStencil &st, const double kb[3],
-                                                    double pb[3]) {
+__device__ __forceinline__ void warp_interp_adjoint(const Geom &g, const float4 *__restrict__ uvr,
+                                                    float *__restrict__ ubar, const double p[3], const double kb[3],
+                                                    int lane, double pb[3]) {
+    LaneStencil s;
+    lane_stencil(g, p[0], p[1], p[2], lane, s);
     double b0 = 0.0, b1 = 0.0, b2 = 0.0;
 #pragma unroll
     for (int h = 0; h < 2; h++)
-        if (st.s.n[h] >= 0) {
-            const long long n = st.s.n[h];
-            atomicAdd(&ubar[4 * n + 0], (float)(st.s.w[h] * kb[0]));
-            atomicAdd(&ubar[4 * n + 1], (float)(st.s.w[h] * kb[1]));
-            atomicAdd(&ubar[4 * n + 2], (float)(st.s.w[h] * kb[2]));
-            const double uk = st.q[h].x * kb[0] + st.q[h].y * kb[1] + st.q[h].z * kb[2];
-            b0 += st.s.dw[h][0] * uk; b1 += st.s.dw[h][1] * uk; b2 += st.s.dw[h][2] * uk;
+        if (s.n[h] >= 0) {
+            const long long n = s.n[h];
+            const float4 q = __ldg(&uvr[n]);
+            atomicAdd(&ubar[4 * n + 0], (float)(s.w[h] * kb[0]));
+            atomicAdd(&ubar[4 * n + 1], (float)(s.w[h] * kb[1]));
+            atomicAdd(&ubar[4 * n + 2], (float)(s.w[h] * kb[2]));
+            const double uk = q.x * kb[0] + q.y * kb[1] + q.z * kb[2];
+            b0 += s.dw[h][0] * uk; b1 += s.dw[h][1] * uk; b2 += s.dw[h][2] * uk;
         }
     pb[0] = warp_sum(b0); pb[1] = warp_sum(b1); pb[2] = warp_sum(b2);
 }
@@ -303,6 +299,11 @@ __device__ __forceinline__ void warp_interp_adjoint(float *__restrict__ ubar, co
 // One warp per vertex.  xa_bar: adjoint of the advected positions; writes
 // X_bar (adjoint of X_t through the advection, overwritten) and adds to ubar.
 // The periodic wrap of the result in x and z is a translation (derivative 1).
+// The reversal of a stage forms its stencil again: 64 registers, 32 warps per
+// multiprocessor.  Kept in registers from the replay (191 registers, 8 warps) the
+// stencils save a microsecond for 162 vertices (13.5 -> 12.4 us) and nothing for
+// 642, and cost from 1284 vertices on (24 -> 25.6 us; 7704: 65 -> 90; 2562 x 148:
+// 3370 -> 4970).
 __global__ void __launch_bounds__(VTX_ADJ_THREADS)
 advect_adjoint_kernel(const Geom g, const double *__restrict__ X, const float4 *__restrict__ uvr,
                       const double *__restrict__ xa_bar, double *__restrict__ X_bar, float *__restrict__ ubar,
@@ -311,13 +312,20 @@ advect_adjoint_kernel(const Geom g, const double *__restrict__ X, const float4 *
     const long long v = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (v >= nv) return;   // uniform over the warp
-    const double p0[3] = {X[v], X[nv + v], X[2 * nv + v]};
-    if (!sane_pos(g, p0[0], p0[1], p0[2])) {
+    double p[4][3], k[3][3];
+    p[0][0] = X[v]; p[0][1] = X[nv + v]; p[0][2] = X[2 * nv + v];
+    if (!sane_pos(g, p[0][0], p[0][1], p[0][2])) {
         if (lane == 0) {
             atomicOr(flags, RBC_FLAG_NONFINITE);
             X_bar[v] = X_bar[nv + v] = X_bar[2 * nv + v] = 0.0;
         }
         return;
+    }
+    const double hs[4] = {0.0, 0.5 * dtM, 0.5 * dtM, dtM};   // stage offsets (ibm.cu:474-498)
+    for (int s = 0; s < 3; s++) {
+        warp_interp(g, uvr, p[s], lane, k[s]);
+        // the forward adds the FP32 stage velocity to the FP64 position
+        for (int c = 0; c < 3; c++) p[s + 1][c] = p[0][c] + (double)(float)k[s][c] * hs[s + 1];
     }
     double xb[3], kb[4][3];
     for (int c = 0; c < 3; c++) {
@@ -325,27 +333,15 @@ advect_adjoint_kernel(const Geom g, const double *__restrict__ X, const float4 *
         xb[c] = a;   // Xa = X + dt (k1 + 2 k2 + 2 k3 + k4) / 6
         kb[0][c] = a * dtM / 6.0; kb[1][c] = a * dtM / 3.0; kb[2][c] = a * dtM / 3.0; kb[3][c] = a * dtM / 6.0;
     }
-    const double hs[4] = {0.0, 0.5 * dtM, 0.5 * dtM, dtM};   // stage offsets (ibm.cu:474-498)
-    StageStencil st[4];
-    double p[3] = {p0[0], p0[1], p0[2]};
-#pragma unroll
-    for (int s = 0; s < 4; s++) {
-        double k[3];
-        warp_interp(g, uvr, p, lane, st[s], k);
-        // the forward adds the FP32 stage velocity to the FP64 position
-        if (s < 3)
-            for (int c = 0; c < 3; c++) p[c] = p0[c] + (double)(float)k[c] * hs[s + 1];
-    }
-#pragma unroll
     for (int s = 3; s >= 0; s--) {
         double pb[3];
-        warp_interp_adjoint(ubar, st[s], kb[s], pb);
+        warp_interp_adjoint(g, uvr, ubar, p[s], kb[s], lane, pb);
         for (int c = 0; c < 3; c++) {
             xb[c] += pb[c];
             if (s > 0) kb[s - 1][c] += hs[s] * pb[c];   // p_s = X + h_s k_s-1
         }
     }
-    if (lane < 3) X_bar[(long long)lane * nv + v] = lane == 0 ? xb[0] : lane == 1 ? xb[1] : xb[2];
+    if (lane < 3) X_bar[(long long)lane * nv + v] = xb[lane];
 }
 
 // ---- spreading, reversed --------------------------------------------------
