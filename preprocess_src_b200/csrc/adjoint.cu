@@ -583,21 +583,25 @@ membrane_adjoint_solve_kernel(const MembraneAdjArgs a)
 
 constexpr int MEM_ADJ_ELEM_THREADS = 128;
 
-// Eight threads per element of any cell: the adjoints of (load on b, load on c,
-// gab) from lambda, q and ds_bar of the element's vertices, contracted with
-// the Jacobian of element_loads (seven dual passes: e1, e2, C).  Thread k < 7 of
-// an element runs the pass of input k (one after another in one thread, the
-// passes left a few cells' elements waiting on seven FP64 chains: 8.8 -> 5.8 us
-// for 1280 elements).
-// Writes the edge adjoints to scratch[7 e + 1 .. 6] and adds dL/dC to cbar.
+// The adjoints of (load on b, load on c, gab) of every element of any cell from
+// lambda, q and ds_bar of its vertices, contracted with the Jacobian of
+// element_loads (seven dual passes: e1, e2, C).  Writes the edge adjoints to
+// scratch[7 e + 1 .. 6] and adds dL/dC to cbar.  LANES = 8: thread k < 7 of an
+// element runs the pass of input k, where a few cells' elements would wait on
+// seven FP64 chains in turn; LANES = 1: one thread runs them one after another,
+// which does the loads and the undifferentiated arithmetic once.  Eight while all
+// their threads are resident at once (118 registers, four blocks per
+// multiprocessor): 1280 elements 10.1 -> 6.8 us, 7680 10.4 -> 8.0, but 15360
+// 10.7 -> 12.6, 122880 30 -> 67 and 757760 143 -> 388.
+template <int LANES>
 __global__ void __launch_bounds__(MEM_ADJ_ELEM_THREADS)
 membrane_adjoint_element_kernel(const MembraneAdjArgs a)
 {
     __shared__ double red[MEM_ADJ_ELEM_THREADS / 32];
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, eg = t >> 3;
-    const int k = (int)(t & 7);
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, eg = t / LANES;
+    const int k0 = (int)(t % LANES);
     double cb = 0.0;
-    if (eg < a.ne && k < 7) {
+    if (eg < a.ne && k0 < 7) {
         const int cell = (int)(eg / a.E), e = (int)(eg - (long long)cell * a.E);
         const long long vb = (long long)cell * a.V;
         double e1[3], e2[3];
@@ -614,16 +618,19 @@ membrane_adjoint_element_kernel(const MembraneAdjArgs a)
         const double bCb[3] = {(double)lc.x - la.x, (double)lc.y - la.y, (double)lc.z - la.z};
         const double4 G = a.gref[eg];
         double *er = a.scratch + 7 * eg;
-        Dual<double> d1[3], d2[3], oB[3], oC[3], og;
-        for (int c = 0; c < 3; c++) {
-            d1[c] = Dual<double>(e1[c], k == c ? 1.0 : 0.0);
-            d2[c] = Dual<double>(e2[c], k == 3 + c ? 1.0 : 0.0);
+#pragma unroll 1
+        for (int k = k0; k < 7; k += LANES) {
+            Dual<double> d1[3], d2[3], oB[3], oC[3], og;
+            for (int c = 0; c < 3; c++) {
+                d1[c] = Dual<double>(e1[c], k == c ? 1.0 : 0.0);
+                d2[c] = Dual<double>(e2[c], k == 3 + c ? 1.0 : 0.0);
+            }
+            const Dual<double> Cd(a.C, k == 6 ? 1.0 : 0.0);
+            element_loads<Dual<double>>(d1, d2, G.x, G.y, G.z, G.w, Cd, a.rgs, a.law, oB, oC, og);
+            double s = og.d * gb;
+            for (int c = 0; c < 3; c++) s += oB[c].d * bBb[c] + oC[c].d * bCb[c];
+            if (k < 6) er[1 + k] = s; else cb = s;
         }
-        const Dual<double> Cd(a.C, k == 6 ? 1.0 : 0.0);
-        element_loads<Dual<double>>(d1, d2, G.x, G.y, G.z, G.w, Cd, a.rgs, a.law, oB, oC, og);
-        double s = og.d * gb;
-        for (int c = 0; c < 3; c++) s += oB[c].d * bBb[c] + oC[c].d * bCb[c];
-        if (k < 6) er[1 + k] = s; else cb = s;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) cb += __shfl_xor_sync(0xffffffffu, cb, o);
@@ -885,8 +892,9 @@ void launch_membrane_adjoint(const MembraneAdjArgs &a, cudaStream_t s)
     case 3: membrane_adjoint_solve_kernel<3><<<a.ncell, T, smem, s>>>(a); break;
     default: membrane_adjoint_solve_kernel<4><<<a.ncell, T, smem, s>>>(a); break;
     }
-    membrane_adjoint_element_kernel<<<(unsigned)((8 * a.ne + MEM_ADJ_ELEM_THREADS - 1) / MEM_ADJ_ELEM_THREADS),
-                                      MEM_ADJ_ELEM_THREADS, 0, s>>>(a);
+    auto blocks = [&](int lanes) { return (unsigned)((lanes * a.ne + MEM_ADJ_ELEM_THREADS - 1) / MEM_ADJ_ELEM_THREADS); };
+    if (a.ne <= 64LL * a.sms) membrane_adjoint_element_kernel<8><<<blocks(8), MEM_ADJ_ELEM_THREADS, 0, s>>>(a);
+    else membrane_adjoint_element_kernel<1><<<blocks(1), MEM_ADJ_ELEM_THREADS, 0, s>>>(a);
     membrane_adjoint_vertex_kernel<<<(unsigned)((a.nv + 127) / 128), 128, 0, s>>>(a);
 }
 

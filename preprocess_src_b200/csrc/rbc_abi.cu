@@ -2935,6 +2935,7 @@ int adjoint_enqueue_reverse(rbc_handle *h, int b, int len, int gb)
             ma.V = h->V; ma.E = h->E; ma.ncell = h->ncell;
             ma.C = h->p.C; ma.rgs = h->cg[0].rgs; ma.law = h->p.law; ma.LX = h->p.LX; ma.LZ = h->p.LZ;
             ma.niter = h->p.solver_iters > 0 ? h->p.solver_iters : DEFAULT_SOLVER_ITERS;
+            ma.sms = h->sms;
             launch_membrane_adjoint(ma, st);
             h->launches += 3;   // the solve, element and vertex passes
             CK_LAUNCH();
@@ -3267,6 +3268,8 @@ int rbc_adjoint_backward(rbc_handle *h, const double *xbar, const double *ybar, 
     if ((rc = d2d(h, h->uvr, a->fin_uvr, 16 * n))) return rc;
     if ((rc = d2d(h, h->U, a->fin_U, 4 * nv3))) return rc;
     if ((rc = d2d(h, h->Fv, a->fin_Fv, 4 * nv3))) return rc;
+    // volume and area are the last recomputed segment's (a binomial sweep's own steps mark them valid)
+    h->metrics_valid = false;
     CK(cudaStreamSynchronize(h->stream));
     return RBC_OK;
 }
@@ -3274,8 +3277,6 @@ int rbc_adjoint_backward(rbc_handle *h, const double *xbar, const double *ybar, 
 int rbc_set_coefficients(rbc_handle *h, double P, double B, double C)
 {
     if (!h || !std::isfinite(P) || !std::isfinite(B) || !std::isfinite(C)) return RBC_ERR_ARG;
-    // volume and area are the last recomputed segment's (a binomial sweep's own steps mark them valid)
-    h->metrics_valid = false;
     RBC_DEVICE_GUARD(h);
     CK(cudaStreamSynchronize(h->stream));
     h->p.P = P; h->p.B = B; h->p.C = C;

@@ -449,6 +449,7 @@ struct MembraneAdjArgs {
     double C, rgs; int law;
     double LX, LZ;
     int niter;
+    int sms;                   // multiprocessors of the device
 };
 void launch_membrane_adjoint(const MembraneAdjArgs &a, cudaStream_t s);
 
