@@ -355,11 +355,9 @@ void launch_spread(const Geom &g, const SpreadArgs &a, cudaStream_t s)
 // same move to about 1e-14).
 // Two lanes do a third fewer instructions per vertex (each lane evaluates the delta
 // weights itself) and hold twice the stencil: 168 registers, three blocks of 128
-// threads per multiprocessor against two of 256 threads.  That is the better trade
-// where blocks queue, four lanes where a block's own latency is the kernel's time:
-// 200 cells of 2562 vertices 118 -> 106 us, 20 of them 19.3 -> 17.4, one cell of 642
-// 10.5 -> 12.2.  Every product and sum over planes is written with its rounding, so
-// both give the same bits.
+// threads per multiprocessor against two of 256 threads: the better trade where blocks
+// queue (advect_two_lanes).  Every product and sum over planes is written with its
+// rounding, so both give the same bits.
 constexpr int ADVECT_VERTICES = 64;   // per pass of a block
 struct Plane16 {
     float u[16], v[16], w[16];
@@ -649,14 +647,26 @@ cudaError_t advect_setup()
     return cudaSuccess;
 }
 
-// more blocks than are resident at once with four lanes (two per multiprocessor)
-static bool advect_two_lanes(long long blocks, int sms) { return blocks > 2LL * sms; }
+// Two lanes per vertex where the blocks of four lanes (two per multiprocessor) take a
+// second round and those of two lanes (three) do not, or where there are so many that
+// rounds no longer count.  Blocks of 161 and 321 vertices, four and two lanes: 300 to 440
+// blocks 27 -> 25 and 39 -> 35 us, 480 31 -> 35 and 46 -> 53, 592 - and 47 -> 57, 800 43 -> 39
+// and 63 -> 62, 1184 54 -> 51 and 86 -> 85, 1600 72 -> 66 and 116 -> 106, 3200 132 -> 117 and
+// 214 -> 194.  Only where the patches are a small part of their cell: one that
+// outgrows the velocity box reads its stencils from L2, which the fewer warps hide less
+// (600 halves of cells 81 -> 97 us; across a periodic x, where the index arithmetic comes on
+// top, 141 -> 252, and eighths 128 -> 145).
+bool advect_two_lanes(const AdvectArgs &a, long long blocks, bool xper)
+{
+    const bool small = xper ? a.patch_most <= 128 || a.npatch >= 16 : a.patch_most <= 256 || a.npatch >= 8;
+    return a.rk == 4 && small && ((blocks > 2LL * a.sms && blocks <= 3LL * a.sms) || blocks > 8LL * a.sms);
+}
 
 void launch_advect(const Geom &g, const AdvectArgs &a, cudaStream_t s)
 {
     if (a.ncell <= 0) return;
     // the lower orders, with a stage or two, keep four lanes
-    const bool two = a.rk == 4 && advect_two_lanes((long long)a.ncell * a.npatch, a.sms);
+    const bool two = advect_two_lanes(a, (long long)a.ncell * a.npatch, g.xper != 0);
     auto k = a.rk == 1 ? (g.xper ? advect_kernel<true, 1, 4> : advect_kernel<false, 1, 4>)
            : a.rk == 2 ? (g.xper ? advect_kernel<true, 2, 4> : advect_kernel<false, 2, 4>)
            : two       ? (g.xper ? advect_kernel<true, 4, 2> : advect_kernel<false, 4, 2>)
@@ -712,10 +722,9 @@ void launch_spread_fused(const FusedLaunch &f, bool xper, cudaStream_t s)
     k<<<f.nblocks, SPREAD_THREADS, SPREAD_SMEM, s>>>(f.dom, f.boff, f.ndom);
 }
 
-void launch_advect_fused(const FusedLaunch &f, bool xper, int sms, cudaStream_t s)
+void launch_advect_fused(const FusedLaunch &f, bool two, bool xper, cudaStream_t s)
 {
     if (f.nblocks <= 0) return;
-    const bool two = advect_two_lanes(f.nblocks, sms);
     auto k = two ? (xper ? advect_fused_kernel<true, 2> : advect_fused_kernel<false, 2>)
                  : (xper ? advect_fused_kernel<true, 4> : advect_fused_kernel<false, 4>);
     k<<<f.nblocks, ADVECT_VERTICES * (two ? 2 : 4), ADVECT_SMEM, s>>>(f.dom, f.boff, f.ndom);

@@ -57,8 +57,10 @@ struct CellGroup {
     double2 *cs0 = nullptr;  // spontaneous angle (cos, sin) per visit [ncell][E][3] (bend_spont), else none
     double *bend_rec = nullptr;   // bending visit records [ncell][E][3][9], allocated when BR != 0
     double *vol0 = nullptr, *gx = nullptr, *vol_out = nullptr, *area_out = nullptr, *cen_out = nullptr;
-    int *patch_off = nullptr, *patch_vtx = nullptr, *patch_stride = nullptr;
-    int npatch = 1;
+    // surface patches at each level (one allocation, patch_vtx): their offsets in patch_vtx and their
+    // number; the spread's level and its lane strides
+    int *patch_vtx = nullptr, *patch_off[PATCH_LEVELS] = {}, *patch_stride = nullptr;
+    int npatch[PATCH_LEVELS] = {}, spread_level = 0;
     int mn = 0;                                       // the reference's per-cell vector length (expand2pow2(3 V))
     double *qi_acc = nullptr, *tp_acc = nullptr;      // output-interval averages [ncell][mn], [ne][2]
     double *vf = nullptr;                             // volume fraction [nint] (ltc->vf, vf2), VOF only
@@ -387,23 +389,22 @@ void initial_volume(const rbc_handle *h, const CellGroup &g, const int *tri, con
 
 // Surface patches for the spread and advection kernels: recursive coordinate
 // bisection of the first cell's initial vertex positions (split along the
-// widest axis at the median until a patch has at most `most` vertices).  The
+// widest axis at the median until a patch has at most patch_most(level)
+// vertices; the patches of a level are the unions of the next one's).  The
 // same vertex sets serve every cell, since all cells share the mesh and a
-// compact patch of the surface stays compact as the membrane moves.  Also a
-// lane stride per patch, near 0.618 of its size and coprime with it, that
-// scatters neighbours across lanes.
-void surface_patches(int V, int most, const double *xr, std::vector<int> &off, std::vector<int> &vtx,
-                     std::vector<int> &stride)
+// compact patch of the surface stays compact as the membrane moves.
+void surface_patches(int V, const double *xr, std::vector<int> (&off)[PATCH_LEVELS], std::vector<int> &vtx)
 {
     vtx.resize(V);
     for (int i = 0; i < V; i++) vtx[i] = i;
-    off.assign(1, 0);
-    std::vector<std::pair<int, int>> stack{{0, V}};
-    std::vector<std::pair<int, int>> leaves;
+    for (auto &o : off) o.assign(1, 0);
+    struct Node { int b, e, level; };   // level: the first one the node's ancestors are not patches of
+    std::vector<Node> stack{{0, V, 0}};   // popped in the order of b
     while (!stack.empty()) {
-        auto [b, e] = stack.back();
+        auto [b, e, level] = stack.back();
         stack.pop_back();
-        if (e - b <= most) { leaves.push_back({b, e}); continue; }
+        while (level < PATCH_LEVELS && e - b <= patch_most(level)) off[level++].push_back(e);
+        if (level == PATCH_LEVELS) continue;
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
         for (int k = b; k < e; k++)
             for (int d = 0; d < 3; d++) { lo[d] = std::min(lo[d], xr[3 * vtx[k] + d]); hi[d] = std::max(hi[d], xr[3 * vtx[k] + d]); }
@@ -412,41 +413,58 @@ void surface_patches(int V, int most, const double *xr, std::vector<int> &off, s
         const int mid = b + (e - b) / 2;
         std::nth_element(vtx.begin() + b, vtx.begin() + mid, vtx.begin() + e,
                          [&](int i, int j) { return xr[3 * i + ax] < xr[3 * j + ax]; });
-        stack.push_back({mid, e});
-        stack.push_back({b, mid});
+        stack.push_back({mid, e, level});
+        stack.push_back({b, mid, level});
     }
-    std::sort(leaves.begin(), leaves.end());
-    stride.clear();
-    for (auto [b, e] : leaves) {
-        off.push_back(e);
-        const int n = e - b;
+}
+
+// A lane stride per patch, near 0.618 of its size and coprime with it, that scatters neighbours across lanes.
+std::vector<int> patch_strides(const std::vector<int> &off)
+{
+    std::vector<int> stride;
+    for (size_t k = 1; k < off.size(); k++) {
+        const int n = off[k] - off[k - 1];
         int s = std::max(1, (int)(0.6180339887 * n)) | 1;
         while (std::gcd(s, n) != 1) s += 2;
         stride.push_back(s);
     }
+    return stride;
 }
 
-// Most vertices of a patch for a population of ncell cells of V vertices.  A
-// block of either kernel takes about 75 ns per vertex of its patch however few
-// blocks run (latency: a few warps per multiprocessor), so a population with
-// few cells is cut into more patches, down to 64 vertices (one pass of the
-// advection's 64 vertices per block), until there are two blocks per
-// multiprocessor.  One cell of 642 vertices in 2, 8, 16 and 32 patches: spread
-// 25, 15.1, 13.1 and 12.9 us, advection 27, 12.9, 11.0 and 10.8 us (events,
-// about 3 us of launch in each), step 71, 46.6, 42.3 and 43.3 us; 9 such cells
-// 74, 52.0, 49.3 and 51.6 us a step; six cells across a periodic x 146, 99, 95
-// and 96 us.  200 cells of 2562 vertices keep 8 patches each.
-int patch_vertices(int ncell, int V, int sms)
+// Patch level of a launch over ncell cells.  A block takes about 75 ns per vertex
+// of its patch however few blocks run (latency: a few warps per multiprocessor), so
+// few cells are cut into more patches while all of them are resident at once (three
+// blocks of either kernel per multiprocessor); beyond that, smaller patches only
+// repeat the boxes' rims.  Spread and advection with both sides of the line measured
+// (us, events, about 3 of launch in each; patches of 321, 161, 81 and 41 of 642
+// vertices): 1 cell 25 + 25, 18 + 16, 18 + 14, 14 + 12; 38 cells 25 + 28, 18 + 18,
+// 16 + 20, 22 + 22 (608 blocks); 60 cells 25 + 27, 18 + 19, 26 + 25 (480 blocks); 29
+// cells of 2562 vertices 25 + 28 in 8 patches each, 29 + 31 in 16 (464 blocks).
+int patch_level(const CellGroup &g, long long ncell, int first, int last, int sms)
 {
-    auto patches = [&](int most) {
-        long long n = 1;
-        for (int v = V; v > most; v = (v + 1) / 2) n *= 2;
-        return n;
-    };
-    int most = MAX_PATCH_VERTICES;
-    while (most > MIN_PATCH_VERTICES && ncell * patches(most) < 2LL * sms) most /= 2;
-    return most;
+    int l = first;
+    while (l < last && ncell * g.npatch[l + 1] <= 3LL * sms) l++;
+    return l;
 }
+
+// The spread's patches are the handle's own whatever batch it is in, since a patch's
+// box has its own fixed-point scale and a batch steps its members bit for bit as they
+// step alone.  So few cells are cut no finer than a batch of many such handles bears:
+// into quarters, or patches of 256 vertices.  Finer, one cell of 642 vertices gains 2 us
+// (161 to 81 vertices) and 4 us (41) of its 46 us step, while a batch of 512 of them pays
+// 31 to 43 and 173 us (capillaries of 32 x 32 x 88 on average 1993 us a step, 2026 with
+// patches of 81, 2169 with 41; ducts of 28 x 28 x 36 943 and 981).
+int spread_last_level(const CellGroup &g)
+{
+    int l = 1;
+    while (l < PATCH_LEVELS - 1 && g.npatch[l] < 4) l++;
+    return l;
+}
+// The advection's do not enter its result, so each launch has its own level.  Halves
+// of a cell (up to 1024 vertices in patches of 512) may outgrow the velocity box, and
+// quarters are the better start: 150 cells of 642 vertices 43 -> 38 us (a radius of
+// 7.8 spacings: 54 -> 41), 600 of them 119 -> 109.
+int advect_first_level(int V) { return V <= 1024 ? 1 : 0; }
 
 // Edge-neighbour visits of fourpoint_bend (stress.cu:448-578, cel->ec from
 // init1.cu:755-795): for element e1, its edge neighbours in increasing
@@ -661,8 +679,8 @@ int build_mask(const rbc_params *p, const int *bc, std::vector<uint32_t> &mask)
 
 void free_group(CellGroup &c)
 {
-    void *cp[] = {c.X, c.Xd, c.gref, c.erec, c.U, c.Fv, c.tri, c.v2e_off, c.v2e, c.nbrp, c.vord, c.visit, c.cs0, c.patch_off,
-                  c.patch_vtx, c.patch_stride, c.vol0, c.vol_out, c.qi_acc, c.tp_acc,
+    void *cp[] = {c.X, c.Xd, c.gref, c.erec, c.U, c.Fv, c.tri, c.v2e_off, c.v2e, c.nbrp, c.vord, c.visit, c.cs0,
+                  c.patch_vtx, c.vol0, c.vol_out, c.qi_acc, c.tp_acc,
                   c.vf, c.bend_rec};
     for (void *q : cp) if (q) cudaFree(q);
     c = CellGroup{};
@@ -727,8 +745,8 @@ int launch_spread_range(rbc_handle *h, CellGroup &g, int c0, int c1, cudaStream_
 {
     SpreadArgs a{};
     a.X = g.X + (size_t)c0 * g.V; a.nv = g.nv; a.V = g.V; a.ncell = c1 - c0; a.Fv = g.Fv + (size_t)c0 * g.V;
-    a.patch_off = g.patch_off; a.patch_vtx = g.patch_vtx; a.patch_stride = g.patch_stride;
-    a.npatch = g.npatch;
+    a.patch_off = g.patch_off[g.spread_level]; a.patch_vtx = g.patch_vtx; a.patch_stride = g.patch_stride;
+    a.npatch = g.npatch[g.spread_level];
     a.F = h->force(); a.mask2d = h->mask2d; a.flags = h->d_flags();
     launch_spread(h->geo, a, st);
     h->launches++;
@@ -806,8 +824,8 @@ SpreadArgs spread_args(rbc_handle *h, CellGroup &g)
 {
     SpreadArgs a{};
     a.X = g.X; a.nv = g.nv; a.V = g.V; a.ncell = g.ncell; a.Fv = g.Fv;
-    a.patch_off = g.patch_off; a.patch_vtx = g.patch_vtx; a.patch_stride = g.patch_stride;
-    a.npatch = g.npatch;
+    a.patch_off = g.patch_off[g.spread_level]; a.patch_vtx = g.patch_vtx; a.patch_stride = g.patch_stride;
+    a.npatch = g.npatch[g.spread_level];
     a.F = h->force(); a.mask2d = h->mask2d; a.flags = h->d_flags();
     return a;
 }
@@ -880,14 +898,19 @@ int launch_lbm_stage(rbc_handle *h, bool reset = true, int acc = LBM_ACC_WRITE)
     return reset ? launch_force_reset_stage(h, h->stream) : RBC_OK;
 }
 
-// the advection kernel's arguments for population g
-AdvectArgs advect_args(rbc_handle *h, CellGroup &g)
+// the advection kernel's arguments for population g, over its patches of the given level
+AdvectArgs advect_args(rbc_handle *h, CellGroup &g, int level)
 {
     AdvectArgs a{};
     a.X = g.X; a.Xd = g.Xd; a.U = g.U; a.uvr = h->uvr; a.nv = g.nv;
-    a.V = g.V; a.ncell = g.ncell; a.patch_off = g.patch_off; a.patch_vtx = g.patch_vtx; a.npatch = g.npatch;
+    a.V = g.V; a.ncell = g.ncell;
+    a.patch_off = g.patch_off[level]; a.patch_vtx = g.patch_vtx; a.npatch = g.npatch[level]; a.patch_most = patch_most(level);
     a.dtM = h->p.dt * h->p.M; a.rk = h->p.rk_order; a.sms = h->sms; a.flags = h->d_flags();
     return a;
+}
+AdvectArgs advect_args(rbc_handle *h, CellGroup &g)
+{
+    return advect_args(h, g, patch_level(g, g.ncell, advect_first_level(g.V), PATCH_LEVELS - 1, h->sms));
 }
 
 // ibm_st2 (ibm.cu:642-694) for every population
@@ -1213,12 +1236,17 @@ int batch_build_fused(rbc_batch *b)
 {
     const int n = (int)b->h.size();
     rbc_handle *h0 = b->h[0];
-    int V = 0;
+    int V = 0, adv_level = 0;
     bool off32 = true;
+    long long cells = 0;
     for (rbc_handle *h : b->h) {
         if (h->cg[0].ncell > 0) V = h->cg[0].V;
         off32 = off32 && (long long)Q * h->geo.nint < (1LL << 31);
+        cells += h->cg[0].ncell;
     }
+    // one advection launch over the cells of all members (which have the same number of vertices)
+    for (rbc_handle *h : b->h)
+        if (h->cg[0].ncell > 0) adv_level = patch_level(h->cg[0], cells, advect_first_level(V), PATCH_LEVELS - 1, h0->sms);
     const int vpt = b->mem_vpt > 0 ? b->mem_vpt : (V > 0 ? membrane_default_vpt(V) : 1);
     const int tpb = b->lbm_threads;
     std::vector<DomainArgs> dom(2 * (size_t)n);
@@ -1237,7 +1265,7 @@ int batch_build_fused(rbc_batch *b)
             D.mem = membrane_args(h, g);
             D.spread = spread_args(h, g);
             D.lbm = lbm_args(h, b->base_cur[i] ^ k);
-            D.adv = advect_args(h, g);
+            D.adv = advect_args(h, g, adv_level);
             D.vol = volume_args(h, g, 1);
             int zpt = b->lbm_planes > 0 ? b->lbm_planes : (h->p.storage == RBC_STORE_F16 ? 4 : 2);
             zpt = std::min(zpt, h->geo.nzc);
@@ -1246,8 +1274,8 @@ int batch_build_fused(rbc_batch *b)
             const long long words = (long long)h->geo.nzc * D.F.wpp;
             constexpr int words_per_block = FUSED_CLEAR_THREADS;   // a warp per 32 words
             const long long cnt[FSTAGES] = {(words + words_per_block - 1) / words_per_block, g.ncell,
-                                            (long long)g.ncell * g.npatch, (long long)D.lbm_bx * D.lbm_gy,
-                                            (long long)g.ncell * g.npatch, g.ncell};
+                                            (long long)g.ncell * D.spread.npatch, (long long)D.lbm_bx * D.lbm_gy,
+                                            (long long)g.ncell * D.adv.npatch, g.ncell};
             for (int st = 0; st < FSTAGES; st++) {
                 boff[((size_t)k * FSTAGES + st) * (n + 1) + i] = acc[st];
                 if ((long long)acc[st] + cnt[st] >= (1LL << 31)) {
@@ -1269,6 +1297,9 @@ int batch_build_fused(rbc_batch *b)
     CKB(cudaMemcpy(d_dom, dom.data(), dbytes, cudaMemcpyHostToDevice));
     CKB(cudaMemcpy(d_boff, boff.data(), obytes, cudaMemcpyHostToDevice));
     const bool fp64 = h0->p.membrane_fp64 != 0, xper = h0->geo.xper != 0;
+    bool two_lanes = false;
+    for (int i = 0; i < n; i++)
+        if (dom[i].adv.ncell > 0) two_lanes = advect_two_lanes(dom[i].adv, nblocks[FS_ADVECT], xper);
     for (int k = 0; k < 2; k++) {
         FusedLaunch f[FSTAGES];
         for (int st = 0; st < FSTAGES; st++)
@@ -1280,7 +1311,7 @@ int batch_build_fused(rbc_batch *b)
         launch_spread_fused(f[FS_SPREAD], xper, b->stream);
         launch_lbm_fused(f[FS_LBM], h0->p.storage, off32, tpb, b->stream);
         launch_clear_bits_fused(f[FS_CLEAR], b->stream);   // the force reset after the read
-        launch_advect_fused(f[FS_ADVECT], xper, h0->sms, b->stream);
+        launch_advect_fused(f[FS_ADVECT], two_lanes, xper, b->stream);
         launch_volume_fused(f[FS_VOLUME], V, b->stream);
         const cudaError_t le = cudaGetLastError();
         const cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
@@ -1373,9 +1404,19 @@ int prepare_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, GroupPrep &
 int upload_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, const GroupPrep &pp)
 {
     int rc;
-    std::vector<int> poff, pvtx, pstride;
-    surface_patches(c.V, patch_vertices(c.ncell, c.V, h->sms), mesh->xr, poff, pvtx, pstride);
-    c.npatch = (int)poff.size() - 1;
+    // the patches in one array: the vertices, each level's offsets, the spread's strides
+    std::vector<int> poff[PATCH_LEVELS], pvtx;
+    surface_patches(c.V, mesh->xr, poff, pvtx);
+    size_t pat[PATCH_LEVELS];
+    for (int l = 0; l < PATCH_LEVELS; l++) {
+        c.npatch[l] = (int)poff[l].size() - 1;
+        pat[l] = pvtx.size();
+        pvtx.insert(pvtx.end(), poff[l].begin(), poff[l].end());
+    }
+    c.spread_level = patch_level(c, c.ncell, 0, spread_last_level(c), h->sms);
+    const std::vector<int> pstride = patch_strides(poff[c.spread_level]);
+    const size_t pst = pvtx.size();
+    pvtx.insert(pvtx.end(), pstride.begin(), pstride.end());
 #define TRYG(x) do { if ((rc = (x))) return rc; } while (0)
     TRYG(dalloc(h, &c.X, 3 * c.nv)); TRYG(dalloc(h, &c.Xd, 3 * c.nv)); TRYG(dalloc(h, &c.gref, c.ne));
     CK(cudaMalloc(&c.erec, (size_t)c.ne * 12 * (h->p.membrane_fp64 ? sizeof(double) : sizeof(float))));
@@ -1391,8 +1432,9 @@ int upload_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, const GroupP
         TRYG(dalloc(h, &c.cs0, pp.cs0.size()));
         CK(cudaMemcpy(c.cs0, pp.cs0.data(), sizeof(double2) * pp.cs0.size(), cudaMemcpyHostToDevice));
     }
-    TRYG(dalloc(h, &c.patch_off, poff.size())); TRYG(dalloc(h, &c.patch_vtx, pvtx.size()));
-    TRYG(dalloc(h, &c.patch_stride, pstride.size()));
+    TRYG(dalloc(h, &c.patch_vtx, pvtx.size()));
+    for (int l = 0; l < PATCH_LEVELS; l++) c.patch_off[l] = c.patch_vtx + pat[l];
+    c.patch_stride = c.patch_vtx + pst;
     TRYG(dalloc(h, &c.vol0, c.ncell));
     // what a caller reads after a step, volume, area and centroid, lies in one block (one copy
     // instead of three), the centroids measured without a correction after them
@@ -1409,9 +1451,7 @@ int upload_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, const GroupP
     CK(cudaMemcpy(c.v2e, pp.packed.data(), 4 * pp.packed.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.nbrp, pp.nbrp6.data(), 2 * 6 * c.V, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.vord, pp.vord.data(), 4 * c.V, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c.patch_off, poff.data(), 4 * poff.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.patch_vtx, pvtx.data(), 4 * pvtx.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c.patch_stride, pstride.data(), 4 * pstride.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.vol0, pp.vol0.data(), 8 * c.ncell, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c.gx, pp.gx.data(), 8 * 3 * c.ncell, cudaMemcpyHostToDevice));
     return RBC_OK;

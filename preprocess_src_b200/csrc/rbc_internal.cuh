@@ -244,10 +244,11 @@ int vof_cg_blocks();
 
 
 
-// Surface patches (spread and advection work units) hold at most this many vertices,
-// and a population with few cells is not cut into patches of fewer than about half MIN.
+// Surface patches (spread and advection work units): at level l a cell is bisected
+// into patches of at most 512 >> l vertices.
+constexpr int PATCH_LEVELS = 4;
 constexpr int MAX_PATCH_VERTICES = 512;
-constexpr int MIN_PATCH_VERTICES = 64;
+constexpr int patch_most(int level) { return MAX_PATCH_VERTICES >> level; }
 
 struct SpreadArgs {
     const double *X; long long nv; int V, ncell;
@@ -267,13 +268,14 @@ struct AdvectArgs {
     long long nv;
     int V, ncell;
     const int *patch_off, *patch_vtx;   // surface patches of the shared mesh
-    int npatch;
+    int npatch, patch_most;    // patches per cell, most vertices of one
     double dtM;                // dt * M
     int rk;                    // RUNGE_KUTTA: 1, 2 or 4 stages
     int sms;                   // multiprocessors of the device
     int *flags;
 };
 void launch_advect(const Geom &g, const AdvectArgs &a, cudaStream_t s);
+bool advect_two_lanes(const AdvectArgs &a, long long blocks, bool xper);   // of a launch of that many blocks like a's
 
 struct MembraneArgs {
     const double *Xd; long long nv, ne;
@@ -518,7 +520,7 @@ void launch_clear_bits_fused(const FusedLaunch &f, cudaStream_t s);   // the for
 void launch_membrane_fused(const FusedLaunch &f, bool fp64, int V, int vpt, cudaStream_t s);   // a block per cell
 void launch_spread_fused(const FusedLaunch &f, bool xper, cudaStream_t s);    // a block per (cell, patch)
 void launch_lbm_fused(const FusedLaunch &f, int storage, bool off32, int threads, cudaStream_t s);
-void launch_advect_fused(const FusedLaunch &f, bool xper, int sms, cudaStream_t s);    // a block per (cell, patch)
+void launch_advect_fused(const FusedLaunch &f, bool two_lanes, bool xper, cudaStream_t s);    // a block per (cell, patch)
 void launch_volume_fused(const FusedLaunch &f, int V, cudaStream_t s);        // a block per cell
 int  membrane_threads(int V, int vpt);     // threads of a membrane block with vpt vertices per thread
 int  membrane_default_vpt(int V);          // the vertices per thread of a one-population launch
