@@ -25,13 +25,15 @@ def _cells(f, n, fp64):
     return case, moved
 
 
-# 1002 vertices: one block; 1212, 2562 and 3242: clusters of four up to 29 cells, of two up to 74 (148 multiprocessors)
+# 1002 vertices: one block; 1212, 2562 and 3242: clusters of four for up to a fifth of the multiprocessors, of two for up to half
 @pytest.mark.parametrize("fp64", [0, 1])
 @pytest.mark.parametrize("f", [10, 11, 16, 18])
 def test_forces_do_not_depend_on_the_number_of_cells(native_lib, oracle_mod, f, fp64):
+    import torch
     from preprocess_src_b200.step import Simulation
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
     first = None
-    for n in (1, 29, 30, 74, 75):
+    for n in (1, sms // 5, sms // 5 + 1, sms // 2, sms // 2 + 1):
         case, x = _cells(f, n, fp64)
         with Simulation(case) as sim:
             xs = [np.tile(x[:, k], n) for k in range(3)]
