@@ -682,8 +682,9 @@ constexpr int VC_ADJ_THREADS = 1024;
 constexpr double VC_COEFF = 0.1;     // COEFF_VOL_CHANGE (volume_correction.cu:14)
 constexpr double VC_TOL = 1.0e-3;    // percent (volume_correction.cu:15)
 
-// One CTA per cell.  Replays the forward correction of the positions Xa (the
-// same unwrap about gx, the same iterations: while |V - V0| / V0 * 100 >= tol,
+// One CTA per cell.  Replays the forward correction of the positions Xa bit for bit
+// (the same unwrap about gx, sums over the same threads, measures, normals and moves:
+// while |V - V0| / V0 * 100 >= tol,
 // every vertex moves by s n_v with s = -0.3 (V - V0) / A and n_v the mean of
 // its elements' unit normals), storing the positions before each move, then
 // reverses the moves: for a move x' = x + s(x) n(x),
@@ -734,9 +735,9 @@ volume_adjoint_kernel(const Geom g, const VolumeAdjArgs a)
         double sv = 0.0, sa = 0.0;
         for (int e = tid; e < E; e += T) {
             int id[3];
-            double A[3], B[3], C[3];
+            double A[3], B[3], C[3], cr[3];
             tri_at(e, id, A, B, C);
-            tri_measure(A, B, C, sv, sa);
+            tri_measure(A, B, C, cr, tri_cross(A, B, C, cr), sv, sa);
         }
         vol = block_sum_r(sv, red) / 18.0;
         area = block_sum_r(sa, red) / 2.0;
@@ -754,11 +755,9 @@ volume_adjoint_kernel(const Geom g, const VolumeAdjArgs a)
         }
         for (int e = tid; e < E; e += T) {
             int id[3];
-            double A[3], B[3], C[3], v1[3], v2[3], cr[3];
+            double A[3], B[3], C[3], cr[3];
             tri_at(e, id, A, B, C);
-            for (int c = 0; c < 3; c++) { v1[c] = B[c] - A[c]; v2[c] = C[c] - A[c]; }
-            cross(v1, v2, cr);
-            const double inv = 1.0 / sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
+            const double inv = 1.0 / tri_cross(A, B, C, cr);
             for (int c = 0; c < 3; c++) er[9 * e + c] = cr[c] * inv;
         }
         for (int k = tid; k < 3 * V; k += T) hist[(long long)moves * 3 * V + k] = p[k];
@@ -772,7 +771,7 @@ volume_adjoint_kernel(const Geom g, const VolumeAdjArgs a)
                 for (int c = 0; c < 3; c++) nn[c] += n[c];
             }
             const double m = s / (double)(k1 - k0);
-            for (int c = 0; c < 3; c++) p[c * V + v] += m * nn[c];
+            for (int c = 0; c < 3; c++) p[c * V + v] = __fma_rn(m, nn[c], p[c * V + v]);
         }
         __syncthreads();
         moves++;
@@ -791,13 +790,12 @@ volume_adjoint_kernel(const Geom g, const VolumeAdjArgs a)
         double sv = 0.0, sa = 0.0, sw = 0.0;
         for (int e = tid; e < E; e += T) {
             int id[3];
-            double A[3], B[3], C[3], v1[3], v2[3], cr[3], W[3];
+            double A[3], B[3], C[3], cr[3], W[3];
             tri_at(e, id, A, B, C);
-            tri_measure(A, B, C, sv, sa);
+            const double norm = tri_cross(A, B, C, cr);
+            tri_measure(A, B, C, cr, norm, sv, sa);
             weight(id, W);
-            for (int c = 0; c < 3; c++) { v1[c] = B[c] - A[c]; v2[c] = C[c] - A[c]; }
-            cross(v1, v2, cr);
-            sw += (cr[0] * W[0] + cr[1] * W[1] + cr[2] * W[2]) / sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
+            sw += (cr[0] * W[0] + cr[1] * W[1] + cr[2] * W[2]) / norm;
         }
         const double vol = block_sum_r(sv, red) / 18.0, area = block_sum_r(sa, red) / 2.0, w = block_sum_r(sw, red);
         const double s = -18.0 * (vol - V0) / area / 6.0 * VC_COEFF;
@@ -808,8 +806,7 @@ volume_adjoint_kernel(const Geom g, const VolumeAdjArgs a)
             tri_at(e, id, A, B, C);
             weight(id, W);
             for (int c = 0; c < 3; c++) { v1[c] = B[c] - A[c]; v2[c] = C[c] - A[c]; }
-            cross(v1, v2, cr);
-            const double inv = 1.0 / sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
+            const double inv = 1.0 / tri_cross(A, B, C, cr);
             double n[3], nW = 0.0;
             for (int c = 0; c < 3; c++) { n[c] = cr[c] * inv; nW += n[c] * W[c]; }
             for (int c = 0; c < 3; c++)

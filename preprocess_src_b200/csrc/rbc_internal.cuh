@@ -338,19 +338,29 @@ struct BendArgs {
 void launch_bend(const BendArgs &a, cudaStream_t s);
 void launch_membrane(const MembraneArgs &a, bool fp64, cudaStream_t s);
 
-// 18 x the volume contribution and 2 x the area of triangle (a, b, c): with
-// c = (b - a) x (c - a), (a + b + c) . c and |c|.  This is the normal form of
-// CalcEleNormal_GPU / CalcVolume (volume_correction.cu:138-200, 246-281:
-// (r . n) dS / 3 with r the centroid, n = c / |c|, dS = |c| / 2) without its
-// divisions; the volume correction and its adjoint's replay both use it.
-__device__ __forceinline__ void tri_measure(const double (&A)[3], const double (&B)[3], const double (&C)[3],
-                                            double &s18v, double &s2a)
+// c = (b - a) x (c - a) of triangle (a, b, c); returns |c|.  18 x the triangle's volume
+// contribution is (a + b + c) . c, twice its area |c| and its normal c / |c|.  This is the
+// normal form of CalcEleNormal_GPU / CalcVolume (volume_correction.cu:138-200, 246-281:
+// (r . n) dS / 3 with r the centroid, n = c / |c|, dS = |c| / 2) without its divisions.
+// Every pass that measures a cell uses these two (the volume correction's first pass, its
+// passes that also form normals, the measuring mode and the adjoint's replay), with no
+// step left to the compiler's contraction: a state is judged the same way by all of them.
+__device__ __forceinline__ double tri_cross(const double (&A)[3], const double (&B)[3], const double (&C)[3], double (&c)[3])
 {
     const double v1x = B[0] - A[0], v1y = B[1] - A[1], v1z = B[2] - A[2];
     const double v2x = C[0] - A[0], v2y = C[1] - A[1], v2z = C[2] - A[2];
-    const double c0 = v1y * v2z - v1z * v2y, c1 = v1z * v2x - v1x * v2z, c2 = v1x * v2y - v1y * v2x;
-    s2a += sqrt(c0 * c0 + c1 * c1 + c2 * c2);
-    s18v += (A[0] + B[0] + C[0]) * c0 + (A[1] + B[1] + C[1]) * c1 + (A[2] + B[2] + C[2]) * c2;
+    c[0] = __fma_rn(v1y, v2z, -__dmul_rn(v1z, v2y));
+    c[1] = __fma_rn(v1z, v2x, -__dmul_rn(v1x, v2z));
+    c[2] = __fma_rn(v1x, v2y, -__dmul_rn(v1y, v2x));
+    return sqrt(__fma_rn(c[2], c[2], __fma_rn(c[0], c[0], __dmul_rn(c[1], c[1]))));
+}
+// adds a triangle's 18 x volume and 2 x area to the sums
+__device__ __forceinline__ void tri_measure(const double (&A)[3], const double (&B)[3], const double (&C)[3],
+                                            const double (&c)[3], double norm, double &s18v, double &s2a)
+{
+    s2a = __dadd_rn(s2a, norm);
+    s18v = __dadd_rn(s18v, __fma_rn(A[2] + B[2] + C[2], c[2],
+                                    __fma_rn(A[0] + B[0] + C[0], c[0], __dmul_rn(A[1] + B[1] + C[1], c[1]))));
 }
 
 struct VolumeArgs {

@@ -50,35 +50,21 @@ __device__ __forceinline__ void block_sum_k(double (&v)[K], double *red) {
     }
 }
 
-// tri_measure of local element e
-__device__ __forceinline__ void ele_measure(const double *__restrict__ p, int V, const int *__restrict__ tri, int e,
-                                            double &s18v, double &s2a)
+// local element e: its part of the cell's measure (MEASURE), its unit normal (NORMAL, CalcEleNormal_GPU)
+template <bool MEASURE, bool NORMAL>
+__device__ __forceinline__ void element(const double *__restrict__ p, int V, const int *__restrict__ tri, int e,
+                                        double (&n)[3], double &s18v, double &s2a)
 {
     const int na = __ldg(&tri[3 * e]), nb = __ldg(&tri[3 * e + 1]), nc = __ldg(&tri[3 * e + 2]);
     const double A[3] = {p[na], p[V + na], p[2 * V + na]};
     const double B[3] = {p[nb], p[V + nb], p[2 * V + nb]};
     const double C[3] = {p[nc], p[V + nc], p[2 * V + nc]};
-    tri_measure(A, B, C, s18v, s2a);
-}
-
-// unit normal of local element e (CalcEleNormal_GPU), and its tri_measure when it is asked for
-template <bool MEASURE>
-__device__ __forceinline__ void ele_normal(const double *__restrict__ p, int V, const int *__restrict__ tri, int e,
-                                           double n[3], double &s18v, double &s2a)
-{
-    const int na = __ldg(&tri[3 * e]), nb = __ldg(&tri[3 * e + 1]), nc = __ldg(&tri[3 * e + 2]);
-    const double ax = p[na], ay = p[V + na], az = p[2 * V + na];
-    const double bx = p[nb], by = p[V + nb], bz = p[2 * V + nb];
-    const double cx = p[nc], cy = p[V + nc], cz = p[2 * V + nc];
-    const double v1x = bx - ax, v1y = by - ay, v1z = bz - az;
-    const double v2x = cx - ax, v2y = cy - ay, v2z = cz - az;
-    const double c0 = v1y * v2z - v1z * v2y, c1 = v1z * v2x - v1x * v2z, c2 = v1x * v2y - v1y * v2x;
-    const double nc_ = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
-    const double inv = 1.0 / nc_;
-    n[0] = c0 * inv; n[1] = c1 * inv; n[2] = c2 * inv;
-    if (MEASURE) {
-        s2a += nc_;
-        s18v += (ax + bx + cx) * c0 + (ay + by + cy) * c1 + (az + bz + cz) * c2;
+    double c[3];
+    const double norm = tri_cross(A, B, C, c);
+    if (MEASURE) tri_measure(A, B, C, c, norm, s18v, s2a);
+    if (NORMAL) {
+        const double inv = 1.0 / norm;
+        for (int k = 0; k < 3; k++) n[k] = c[k] * inv;
     }
 }
 
@@ -132,12 +118,15 @@ __device__ __forceinline__ void volume_body(const Geom &g, const VolumeArgs &a, 
         if (cached && it > 0) {
             for (int e = tid; e < E; e += T) {
                 double n[3];
-                ele_normal<true>(p, V, a.tri, e, n, s[0], s[1]);
+                element<true, true>(p, V, a.tri, e, n, s[0], s[1]);
                 nrm[e] = n[0]; nrm[E + e] = n[1]; nrm[2 * E + e] = n[2];
             }
         } else {
 #pragma unroll 2
-            for (int e = tid; e < E; e += T) ele_measure(p, V, a.tri, e, s[0], s[1]);
+            for (int e = tid; e < E; e += T) {
+                double n[3];
+                element<true, false>(p, V, a.tri, e, n, s[0], s[1]);
+            }
         }
         block_sum_k<2>(s, red);
         vol = s[0] / 18.0;
@@ -151,7 +140,7 @@ __device__ __forceinline__ void volume_body(const Geom &g, const VolumeArgs &a, 
             if (it == 1) {
                 for (int e = tid; e < E; e += T) {
                     double n[3], u0, u1;
-                    ele_normal<false>(p, V, a.tri, e, n, u0, u1);
+                    element<false, true>(p, V, a.tri, e, n, u0, u1);
                     nrm[e] = n[0]; nrm[E + e] = n[1]; nrm[2 * E + e] = n[2];
                 }
                 __syncthreads();
@@ -164,29 +153,28 @@ __device__ __forceinline__ void volume_body(const Geom &g, const VolumeArgs &a, 
                     n0 += nrm[e]; n1 += nrm[E + e]; n2 += nrm[2 * E + e];
                 }
                 const double m = move / (double)(k1 - k0);
-                p[v] += m * n0; p[V + v] += m * n1; p[2 * V + v] += m * n2;
+                p[v] = __fma_rn(m, n0, p[v]); p[V + v] = __fma_rn(m, n1, p[V + v]); p[2 * V + v] = __fma_rn(m, n2, p[2 * V + v]);
             }
             __syncthreads();
         } else {   // a cell too large for the normals: each vertex forms those of its elements
-            double disp[4][3];
+            double sum[4][3], w[4];
             for (int m = 0; m < 4; m++) {
                 const int v = tid + m * T;
-                disp[m][0] = disp[m][1] = disp[m][2] = 0.0;
+                sum[m][0] = sum[m][1] = sum[m][2] = 0.0;
                 if (v >= V) continue;
                 const int k0 = __ldg(&a.v2e_off[v]), k1 = __ldg(&a.v2e_off[v + 1]);
                 for (int k = k0; k < k1; k++) {
                     double n[3], u0, u1;
-                    ele_normal<false>(p, V, a.tri, v2e_elem(__ldg(&a.v2e[k])), n, u0, u1);
-                    disp[m][0] += n[0]; disp[m][1] += n[1]; disp[m][2] += n[2];
+                    element<false, true>(p, V, a.tri, v2e_elem(__ldg(&a.v2e[k])), n, u0, u1);
+                    for (int c = 0; c < 3; c++) sum[m][c] += n[c];
                 }
-                const double w = move / (double)(k1 - k0);
-                for (int c = 0; c < 3; c++) disp[m][c] *= w;
+                w[m] = move / (double)(k1 - k0);
             }
             __syncthreads();
             for (int m = 0; m < 4; m++) {
                 const int v = tid + m * T;
                 if (v >= V) continue;
-                p[v] += disp[m][0]; p[V + v] += disp[m][1]; p[2 * V + v] += disp[m][2];
+                for (int c = 0; c < 3; c++) p[c * V + v] = __fma_rn(w[m], sum[m][c], p[c * V + v]);
             }
             __syncthreads();
         }
