@@ -1809,12 +1809,15 @@ static double *mapped(double *p, size_t n)
     return start <= at && at + n * sizeof(double) <= start + size ? (double *)dev : nullptr;
 }
 
-// Results of up to this many bytes go to page-locked buffers from the kernel that
-// lays them out, without a staging copy per array (several us each on the copy queue,
-// 13 for a population and its fields); larger results take the staged copies, which
-// keep the host link busier than a kernel's stores.  Cells and fields of a 64 x 32 x 32
-// duct 245 -> 121 us, of an 8.2 MB result 823 -> 740 us.
-constexpr size_t EXPORT_DIRECT_BYTES = 16u << 20;
+// Results go to page-locked buffers from the kernel that lays them out where that saves
+// more than it costs: staging costs a copy per array (about 3 us each on the copy queue,
+// which the kernel's own launch outweighs for three of them) and a conversion for most of
+// a population's arrays, the kernel's stores run at 52 GB/s against the copies' 55.  So
+// up to 2 MB per array, the first three of a population's not counted.  Staged and direct:
+// the four fields 51 -> 40 us (1 MB), 110 -> 102 (4 MB), 182 -> 180 (8 MB), 256 -> 260 (12
+// MB), 1226 -> 1294 (64 MB); all arrays of a population 76 -> 31 (0.2 MB), 353 -> 326 (15 MB),
+// 1215 -> 1250 (61 MB); positions alone 21 -> 21 (0.1 MB), 90 -> 94 (4 MB).
+constexpr size_t EXPORT_DIRECT_BYTES = 2u << 20;
 
 int rbc_export_ref_lattice(rbc_handle *h, double *fn, double *dn, double *un, double *vn, double *wn)
 {
@@ -1823,7 +1826,7 @@ int rbc_export_ref_lattice(rbc_handle *h, double *fn, double *dn, double *un, do
     const bool macro = dn || un || vn || wn;
     if (!fn && !macro) return RBC_OK;
     const size_t n = (size_t)h->nref_nodes;
-    if (!fn && 8 * 4 * n <= EXPORT_DIRECT_BYTES) {
+    if (!fn && 8 * n <= EXPORT_DIRECT_BYTES) {
         double *m[4] = {mapped(dn, n), mapped(un, n), mapped(vn, n), mapped(wn, n)};
         if (m[0] && m[1] && m[2] && m[3]) {
             launch_export_lattice(h->geo, h->p.storage, h->g[h->cur], h->mask2d, h->uvr, h->inv_scale, nullptr, m[0], m[1],
@@ -2030,9 +2033,11 @@ static int export_cells(rbc_handle *h, CellGroup &G, double *x, double *y, doubl
     const int N = G.ncell;
     cudaStream_t s = h->stream;
     double *outs[6] = {u, v, w, fx, fy, fz};
-    if (8 * (size_t)(12 * nv + 3 * N) <= EXPORT_DIRECT_BYTES) {
+    double *const in[3] = {x, y, z};
+    size_t arrays = (xd != nullptr) + (gxo != nullptr), values = (xd ? 3 * (size_t)nv : 0) + (gxo ? 3 * (size_t)N : 0);
+    for (double *q : {x, y, z, u, v, w, fx, fy, fz}) { arrays += q != nullptr; values += q ? (size_t)nv : 0; }
+    if (arrays > 3 && 8 * values <= (arrays - 3) * EXPORT_DIRECT_BYTES) {
         CellExport o{};
-        double *const in[3] = {x, y, z};
         bool all = true;
         auto map = [&](double *p, size_t n) { double *m = mapped(p, n); all = all && (m || !p); return m; };
         for (int c = 0; c < 3 && all; c++) o.x[c] = map(in[c], nv);
