@@ -63,7 +63,9 @@ constexpr int MEM_MAX_THREADS = 1024;
 
 // pos 24V (then the solve's two d-buffers, 3 x V floats each), 8V unused, coef 24V
 int membrane_smem_bytes(int V) { return 56 * V; }
-// what the vertices per cell are limited by
+// Bytes per vertex that limit the vertices per cell (3418 in 227 KB).  More than this pass
+// asks for: four vertices per thread of at most 896 threads end at 3584, and the volume
+// correction and its adjoint (24 to 48 bytes per vertex) beyond that.
 int membrane_limit_bytes(int V) { return 68 * V; }
 
 __device__ __forceinline__ double mimage(double d, double L) {
@@ -410,7 +412,7 @@ static void launch_real(const MembraneArgs &a, cudaStream_t s)
     if (fits(1, mem_max_threads<1>())) launch_vpt<Real, 1>(a, s);
     else if (fits(2, mem_max_threads<2>())) launch_vpt<Real, 2>(a, s);
     else if (fits(3, mem_max_threads<3>())) launch_vpt<Real, 3>(a, s);
-    else launch_vpt<Real, 4>(a, s);   // V <= 3418 (shared-memory limit) fits 4 x 896
+    else launch_vpt<Real, 4>(a, s);   // V <= 3418 (membrane_limit_bytes) fits 4 x 896
 }
 
 cudaError_t set_max_dyn_smem(const void *kernel, int optin, int *granted);

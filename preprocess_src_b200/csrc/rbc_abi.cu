@@ -1542,6 +1542,12 @@ static int import_lattice_pipelined(rbc_handle *h, const double *fn, const WallV
 static cudaError_t cell_io_setup();
 static int ensure_cell_staging(rbc_handle *h, const CellGroup &G);
 
+constexpr int MEM_SMEM_MAX = 227 * 1024;   // dynamic shared memory a block can have
+static std::string too_many_vertices(int bytes)
+{
+    return "more vertices per cell than supported (max " + std::to_string(bytes / membrane_limit_bytes(1)) + ")";
+}
+
 int rbc_create(const rbc_params *p, const rbc_mesh *mesh, const int *bc, rbc_handle **out)
 {
     g_create_error.clear();
@@ -1556,8 +1562,8 @@ int rbc_create(const rbc_params *p, const rbc_mesh *mesh, const int *bc, rbc_han
     if (cells) {
         if (mesh->vertex < 4 || mesh->element < 4 || !mesh->tri || !mesh->xr)
             return fail(nullptr, RBC_ERR_ARG, "mesh needs vertex, element >= 4, tri and xr");
-        if (membrane_limit_bytes(mesh->vertex) > 227 * 1024 || mesh->vertex > 4096)
-            return fail(nullptr, RBC_ERR_UNSUPPORTED, "more vertices per cell than one CTA holds (max 3874)");
+        if (mesh->vertex > MEM_SMEM_MAX || membrane_limit_bytes(mesh->vertex) > MEM_SMEM_MAX)
+            return fail(nullptr, RBC_ERR_UNSUPPORTED, too_many_vertices(MEM_SMEM_MAX));
         if (mesh->element >= (1 << 24)) return fail(nullptr, RBC_ERR_UNSUPPORTED, "too many elements per cell");
     }
     rbc_handle *h = new (std::nothrow) rbc_handle();
@@ -1608,7 +1614,7 @@ int rbc_create(const rbc_params *p, const rbc_mesh *mesh, const int *bc, rbc_han
         if (!e) e = (int)cell_io_setup();
         if (e) { h->err = std::string("kernel attributes: ") + cudaGetErrorString((cudaError_t)e); return bail(RBC_ERR_CUDA); }
         if (cells && membrane_limit_bytes(mesh->vertex) > mem_max) {
-            h->err = "more vertices per cell than one CTA's shared memory holds";
+            h->err = too_many_vertices(mem_max);
             return bail(RBC_ERR_UNSUPPORTED);
         }
     }
@@ -3536,8 +3542,8 @@ int rbc_add_wbc(rbc_handle *h, const rbc_mesh *mesh, double rgs, double br)
     if (h->ngroups > 1) return fail(h, RBC_ERR_STATE, "the white cells are already set");
     if (mesh->vertex < 4 || mesh->element < 4 || !mesh->tri || !mesh->xr)
         return fail(h, RBC_ERR_ARG, "mesh needs vertex, element >= 4, tri and xr");
-    if (membrane_limit_bytes(mesh->vertex) > 227 * 1024 || mesh->vertex > 4096)
-        return fail(h, RBC_ERR_UNSUPPORTED, "more vertices per cell than one CTA holds (max 3874)");
+    if (mesh->vertex > MEM_SMEM_MAX || membrane_limit_bytes(mesh->vertex) > MEM_SMEM_MAX)
+        return fail(h, RBC_ERR_UNSUPPORTED, too_many_vertices(MEM_SMEM_MAX));
     if (mesh->element >= (1 << 24)) return fail(h, RBC_ERR_UNSUPPORTED, "too many elements per cell");
     if (!(rgs > 0.0) || !std::isfinite(rgs) || !std::isfinite(br)) return fail(h, RBC_ERR_ARG, "rgs must be > 0 and br finite");
     CK(cudaStreamSynchronize(h->stream));

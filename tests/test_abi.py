@@ -86,6 +86,17 @@ def test_rejects_broken_mesh(native_lib):
     assert _create(case)[0] == N.RBC_ERR_TOPOLOGY
 
 
+@pytest.mark.parametrize("vertex,refused", [(3418, False), (3419, True), (4096, True), (5000, True), (63161284, True)])
+def test_vertices_per_cell_limit(native_lib, vertex, refused):
+    """The limit that the message names is the one that is applied."""
+    case = configs.small_duct()
+    case.vertex = vertex   # the connectivity stays the small cell's: no closed mesh of that many vertices
+    case.xr = np.zeros(3 * min(vertex, 5000))   # (refused before it is read)
+    rc, msg = _create(case)
+    assert (rc == N.RBC_ERR_UNSUPPORTED) == refused, (rc, msg)
+    assert ("(max 3418)" in msg) == refused
+
+
 @pytest.mark.skipif(_cuda_present(), reason="checks the no-device path")
 def test_no_device_is_reported(native_lib):
     rc, msg = _create(configs.small_duct())
