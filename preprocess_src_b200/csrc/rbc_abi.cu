@@ -450,14 +450,15 @@ int patch_level(const CellGroup &g, long long ncell, int first, int last, int sm
 // The spread's patches are the handle's own whatever batch it is in, since a patch's
 // box has its own fixed-point scale and a batch steps its members bit for bit as they
 // step alone.  So few cells are cut no finer than a batch of many such handles bears:
-// into quarters, or patches of 256 vertices.  Finer, one cell of 642 vertices gains 2 us
-// (161 to 81 vertices) and 4 us (41) of its 46 us step, while a batch of 512 of them pays
-// 31 to 43 and 173 us (capillaries of 32 x 32 x 88 on average 1993 us a step, 2026 with
-// patches of 81, 2169 with 41; ducts of 28 x 28 x 36 943 and 981).
+// into eight patches, or patches of 256 vertices.  One cell of 642 vertices in patches of
+// 321, 161, 81 and 41: spread 25, 18, 16 and 14 us alone; a batch of 512 of them 2040,
+// 1993, 2026 and 2169 us a step in capillaries of 32 x 32 x 88 on average, 949, 943, 981
+// and 1040 in ducts of 28 x 28 x 36; 64 members of 2562 vertices 387 us in patches of 321 and
+// of 161, 397 in patches of 81.
 int spread_last_level(const CellGroup &g)
 {
     int l = 1;
-    while (l < PATCH_LEVELS - 1 && g.npatch[l] < 4) l++;
+    while (l < PATCH_LEVELS - 1 && g.npatch[l] < 8) l++;
     return l;
 }
 // The advection's do not enter its result, so each launch has its own level.  Halves
