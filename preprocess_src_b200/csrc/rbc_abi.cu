@@ -2695,7 +2695,7 @@ int rbc_batch_launch_count(const rbc_batch *b, long long *count)
 // and reversal are CUDA graphs, captured once per (store, buffer parity,
 // length) and replayed.  Device memory: nsteps / K + 1 checkpoints
 // (4 Q B per node + 48 B per vertex) and 2 K steps of stored stages
-// (104 B per node + 84 B per vertex).
+// (104 B per node + 60 B per vertex, and fem->xd once per store).
 
 // Binomial checkpointing (rbc_adjoint_record_binomial): the run is cut into
 // units of `unit` steps and reversed unit by unit under the schedule of

@@ -513,7 +513,32 @@ constexpr double MG_OMEGA = 0.8;   // damped-Jacobi smoothing weight
 constexpr int MG_COARSE_SWEEPS = 40;
 constexpr int MG_COARSE_SMEM = 512;   // nodes of a coarsest level swept in shared memory (the coarsening's target)
 
-// The coarsest level: Jacobi sweeps from 0 in block 0.  Each sweep is a short
+// The coarsest level of a lattice whose extents do not coarsen below MG_COARSE_SMEM nodes
+// (an odd periodic length stays as it is: 48 x 48 columns end above 512 nodes from a length of
+// 57 on, twice an odd one from 114): Jacobi sweeps from 0 in block 0, from
+// global memory, x and y alternating.  These sweeps are then nearly all of the solve (48 x 48
+// columns, per iteration: length 96 56 us, 131 244, 255 405).  A function of its own: inlined
+// into the kernel its loop is compiled worse (131 318 us, 255 544).
+__device__ __noinline__ void coarse_sweeps_global(const MgLevel &C)
+{
+    const unsigned nc = (unsigned)C.n, ncc = (unsigned)(C.nx * C.ny);
+    for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) C.y[i] = 0.0;
+    __syncthreads();
+    double *src = C.y, *dst = C.x;
+    for (int sw = 0; sw < MG_COARSE_SWEEPS; sw++) {
+        for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) {
+            const unsigned Z = i / ncc, rc = i - Z * ncc, Y = rc / (unsigned)C.nx, X = rc - Y * (unsigned)C.nx;
+            const double id = C.coef[6 * ncc + rc];
+            dst[i] = id != 0.0 ? src[i] + MG_OMEGA * (C.b[i] - apply_level(C, src, i, (int)X, (int)Y, (int)Z)) * id : 0.0;
+        }
+        __syncthreads();
+        double *t = src; src = dst; dst = t;
+    }
+    if (src != C.y)
+        for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) C.y[i] = src[i];
+}
+
+// The coarsest level otherwise: Jacobi sweeps from 0 in block 0.  Each sweep is a short
 // dependent step (seven loads, one barrier), so it runs from shared memory with
 // each thread's rows in registers.
 __device__ void coarse_sweeps(const MgLevel &C)
@@ -570,21 +595,7 @@ __device__ void coarse_sweeps(const MgLevel &C)
         }
         return;
     }
-    // a lattice whose extents do not coarsen that far: from global memory (x and y alternate)
-    for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) C.y[i] = 0.0;
-    __syncthreads();
-    double *src = C.y, *dst = C.x;
-    for (int sw = 0; sw < MG_COARSE_SWEEPS; sw++) {
-        for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) {
-            const unsigned Z = i / ncc, rc = i - Z * ncc, Y = rc / (unsigned)C.nx, X = rc - Y * (unsigned)C.nx;
-            const double id = C.coef[6 * ncc + rc];
-            dst[i] = id != 0.0 ? src[i] + MG_OMEGA * (C.b[i] - apply_level(C, src, i, (int)X, (int)Y, (int)Z)) * id : 0.0;
-        }
-        __syncthreads();
-        double *t = src; src = dst; dst = t;
-    }
-    if (src != C.y)
-        for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) C.y[i] = src[i];
+    coarse_sweeps_global(C);
 }
 
 // z = M r: one symmetric V-cycle (one damped-Jacobi sweep from 0 before and
