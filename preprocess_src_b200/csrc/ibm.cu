@@ -621,7 +621,8 @@ advect_body(const Geom &g, double *__restrict__ X, double *__restrict__ Xd, floa
     }
 }
 
-// resident blocks per multiprocessor the register allocation must allow
+// resident blocks per multiprocessor the register allocation must allow (two lanes: 168 registers; the
+// forms across a periodic x and in a fused batch spill 120 to 230 bytes at that)
 constexpr int advect_min_blocks(int lanes) { return lanes == 2 ? 3 : 2; }
 
 template <bool XPER, int RK, int LANES>

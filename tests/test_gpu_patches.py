@@ -1,10 +1,10 @@
 """Spread and advection over the surface patches a population is cut into.
 
-The patch size follows the number of cells (more and smaller patches for few
-cells), so the same step is checked against the FP64 oracle for cells that stay
-whole, for the smallest patches, and for populations on both sides of the
-two-blocks-per-multiprocessor line.  Tolerances per step as in
-test_gpu_parity.py."""
+The patches follow the number of cells (each launch takes the smallest ones
+whose blocks are resident at once, the spread down to eight patches a cell), so
+the same step is checked against the FP64 oracle for cells that stay whole, for
+the smallest patches, and for populations on both sides of the lines.
+Tolerances per step as in test_gpu_parity.py."""
 import numpy as np
 import pytest
 
@@ -14,7 +14,7 @@ from tests.test_gpu_parity import comp, rel_l2
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("subdiv,ncell,flow", [(1, 1, 24), (2, 1, 24), (3, 2, 40), (4, 1, 32), (2, 70, 200)])
+@pytest.mark.parametrize("subdiv,ncell,flow", [(1, 1, 24), (2, 1, 24), (3, 2, 40), (4, 1, 32), (2, 70, 200), (3, 30, 200), (3, 60, 200)])
 def test_step_matches_oracle(native_lib, oracle_mod, subdiv, ncell, flow):
     from preprocess_src_b200.step import Simulation
     if ncell <= 2:
