@@ -649,8 +649,8 @@ cudaError_t advect_setup()
 }
 
 // Two lanes per vertex where the blocks of four lanes (two per multiprocessor) take a
-// second round and those of two lanes (three) do not, or where there are so many that
-// rounds no longer count.  Blocks of 161 and 321 vertices, four and two lanes: 300 to 440
+// second wave and those of two lanes (three) do not, or where there are so many that
+// waves no longer count.  Blocks of 161 and 321 vertices, four and two lanes: 300 to 440
 // blocks 27 -> 25 and 39 -> 35 us, 480 31 -> 35 and 46 -> 53, 592 - and 47 -> 57, 800 43 -> 39
 // and 63 -> 62, 1184 54 -> 51 and 86 -> 85, 1600 72 -> 66 and 116 -> 106, 3200 132 -> 117 and
 // 214 -> 194.  Only where the patches are a small part of their cell: one that
