@@ -452,9 +452,9 @@ int patch_level(const CellGroup &g, long long ncell, int first, int last, int sm
 // step alone.  So few cells are cut no finer than a batch of many such handles bears:
 // into eight patches, or patches of 256 vertices.  One cell of 642 vertices in patches of
 // 321, 161, 81 and 41: spread 25, 18, 16 and 14 us alone; a batch of 512 of them 2040,
-// 1993, 2026 and 2169 us a step in capillaries of 32 x 32 x 88 on average, 949, 943, 981
-// and 1040 in ducts of 28 x 28 x 36; 64 members of 2562 vertices 387 us in patches of 321 and
-// of 161, 397 in patches of 81.
+// 1993, 2026 and 2169 us a step in capillaries of 32 x 32 x 88 on average (the last with the
+// advection in patches of 41 as well), 949, 943 and 981 in ducts of 28 x 28 x 36; 64 members
+// of 2562 vertices 387 us in patches of 321 and of 161, 397 in patches of 81.
 int spread_last_level(const CellGroup &g)
 {
     int l = 1;
