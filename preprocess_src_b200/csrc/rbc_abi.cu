@@ -450,16 +450,17 @@ int patch_level(const CellGroup &g, long long ncell, int first, int last, int sm
 // The spread's patches are the handle's own whatever batch it is in, since a patch's
 // box has its own fixed-point scale and a batch steps its members bit for bit as they
 // step alone.  So few cells are cut no finer than a batch of many such handles bears:
-// into eight patches, or patches of 256 vertices.  One cell of 642 vertices in patches of
-// 321, 161, 81 and 41: spread 25, 18, 16 and 14 us alone; a batch of 512 of them 2040,
-// 1993, 2026 and 2169 us a step in capillaries of 32 x 32 x 88 on average (the last with the
-// advection in patches of 41 as well), 949, 943 and 981 in ducts of 28 x 28 x 36; 64 members
-// of 2562 vertices 387 us in patches of 321 and of 161, 397 in patches of 81.
-int spread_last_level(const CellGroup &g)
+// into patches of 128 vertices (whole cells of up to 256 vertices: of 64), or of 256 where
+// the lattice has fewer than 20 nodes per vertex and the spread would weigh most.  One cell
+// of 642 vertices in patches of 321, 161, 81 and 41: spread 25, 18, 16 and 14 us alone; a
+// batch of 512 of them 2040, 1993, 2026 and 2169 us a step in capillaries of 32 x 32 x 88 on
+// average (the last with the advection in patches of 41 as well), 949, 943 and 981 in ducts
+// of 28 x 28 x 36 (44 nodes per vertex).  Members of 2562 vertices in patches of 321, 161 and
+// 81: 64 on 48 x 40 x 40 (30 nodes per vertex) 387, 387 and 397 us, 200 on 36 x 28 x 28 (11)
+// 661, 675 and 732.
+int spread_last_level(const CellGroup &g, long long nodes)
 {
-    int l = 1;
-    while (l < PATCH_LEVELS - 1 && g.npatch[l] < 8) l++;
-    return l;
+    return g.V <= 256 ? 3 : nodes >= 20 * g.nv ? 2 : 1;
 }
 // The advection's do not enter its result, so each launch has its own level.  Halves
 // of a cell (up to 1024 vertices in patches of 512) may outgrow the velocity box, and
@@ -1414,7 +1415,7 @@ int upload_group(rbc_handle *h, CellGroup &c, const rbc_mesh *mesh, const GroupP
         pat[l] = pvtx.size();
         pvtx.insert(pvtx.end(), poff[l].begin(), poff[l].end());
     }
-    c.spread_level = patch_level(c, c.ncell, 0, spread_last_level(c), h->sms);
+    c.spread_level = patch_level(c, c.ncell, 0, spread_last_level(c, h->geo.nint), h->sms);
     const std::vector<int> pstride = patch_strides(poff[c.spread_level]);
     const size_t pst = pvtx.size();
     pvtx.insert(pvtx.end(), pstride.begin(), pstride.end());
